@@ -336,7 +336,11 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
     g.m = m;
     g.u_num = hg->u_num;
     uint32_t maxd = 0;
-    for (uint32_t x = 0; x < n; x++) maxd = hg->degrees[x] > maxd ? hg->degrees[x] : maxd;
+    for (uint32_t x = 0; x < n; x++) {
+        const uint32_t d = hg->degrees[x];
+        maxd = d > maxd ? d : maxd;
+        if (d) g.tab_buckets += bt_row_buckets(d);
+    }
     g.max_deg = maxd;
 
     // persistent arrays

@@ -90,11 +90,16 @@ struct DevGraph {
     uint32_t *hub_mask = nullptr;
     uint2 *hub_pool = nullptr;
     uint64_t hub_slots = 0;
+    uint64_t tab_buckets = 0;  // row table buckets of the peel (32 bytes each)
     // batched arena: ranks are grouped by graph; seg_base[r] = first rank of
     // r's graph (NULL for one graph); cnt_span = vertices of the largest graph
     uint32_t *seg_base = nullptr;
     uint32_t cnt_span = 0;
 };
+
+// 32-byte buckets of the peel's hash table of a row of d edges: 1.5 slots per
+// edge, at least one of them free.
+__host__ __device__ inline uint32_t bt_row_buckets(uint32_t d) { return (d + (d >> 1) + 4) >> 2; }
 
 // ---------------------------------------------------------------------------
 // device context
@@ -130,15 +135,15 @@ struct bt_ctx {
     uint64_t prof[8] = {0};   // msp: SM cycles per CTA by step (task, stage, slice, probe, hits, flush, barrier, other)
     cudaEvent_t ev[8] = {};
 
-    // msp task schedule (0 = built-in value): min grain, tasks per CTA, local-plan limit
+    // msp task schedule (0 = built-in value): positions per task, chunks per CTA, whole-plan limit
     uint32_t msp_schedule[3] = {0, 0, 0};
     uint64_t arena_edges = 1ull << 28;  // batched calls: edges per arena, at most
     uint32_t peel_ctas = 0;             // CTAs of the peeling kernel (0 = one per SM)
 };
 
 // Default msp task schedule (bt_ctx_set_msp_schedule with 0 picks these):
-// probe positions per task at least, tasks per CTA, local-plan limit.
-constexpr uint32_t kMspMinGrain = 2048;
+// probe positions per task, frontier chunks per CTA, whole-plan limit.
+constexpr uint32_t kMspMinGrain = 64;
 constexpr uint32_t kMspTasksPerCta = 2;
 constexpr uint32_t kMspLocalPlan = 512;
 

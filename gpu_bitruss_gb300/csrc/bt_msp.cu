@@ -22,28 +22,52 @@
 // GB300 design: one cooperative persistent kernel runs the whole level /
 // sub-round loop on the device (the reference pays 3 host syncs and ~9m bytes
 // of copies per sub-round, :527-533).
+//
+// What bounds it: the chain.  A decomposition is tens of thousands of
+// sub-rounds that depend on one another, most of them of 10^3 to 10^5 row
+// positions, so a sub-round's time is the number of dependent L2 round trips
+// (430 cycles each) and barriers on its longest path, not bandwidth.  Measured
+// per sub-round, against staging the anchor row in shared memory and walking
+// equal shares of probe positions by whole CTAs: Chung-Lu graphs of 10k / 200k
+// / 1M edges 6.7 / 8.0 / 10.7 us (19.4 / 21.8 / 28.7 before), the 20M-edge one
+// 45 us (87), hub-skewed graphs of 200k / 2M edges 12.2 / 31 us (28.5 / 49).
+// What follows from that:
 //  * Edge state is one stamp per edge: enter[e] = the index of the sub-round
 //    whose frontier e joined (0: not yet).  In sub-round r an edge is in the
 //    frontier iff enter == r and processed iff 0 < enter < r, so "mark the
 //    frontier processed, promote the next frontier" costs nothing: the thread
 //    that pushes an edge to the next frontier stamps it r+1 and records its
 //    result (L).  A sub-round therefore needs one grid barrier.
+//  * Every row has a hash table (neighbour -> edge id) over its live edges,
+//    rebuilt at each row compaction, so a (mid, anchor) pair is intersected
+//    from its shorter row with one table read per position and nothing has to
+//    be staged first.
+//  * A frontier of up to 32 edges is planned inside the barrier: its entries
+//    are loaded with the control words, whoever pushed them having written
+//    their endpoints beside them.  Up to 512 edges every CTA plans the whole
+//    frontier; more than that are cut into chunks that CTAs take from a
+//    counter.
+//  * A task is a warp on a block of 32 pivot slots (mids), one per lane, or on
+//    an equal part of the block's positions; the positions of the block's live
+//    mids lie end to end and are taken 32 at a time, so lanes stay full
+//    whatever the rows' lengths.  Tasks are dealt to the CTAs round robin and
+//    taken by their warps one by one.  No block barriers.
+//  * Only one warp per CTA reads what all of them need (control words, the
+//    frontier): the same word read by every warp of the grid at once is served
+//    one request at a time and costs more than the rest of the plan.
 //  * Frontier discovery uses two support buckets: "near" holds the live
 //    edges with support < hi, "far" the rest.  A level scans only the near
 //    list; when it runs dry the far list is split again.  A decrement that
-//    crosses hi appends the edge to near.
-//  * Every CTA plans a small frontier itself in shared memory (orientation of
-//    each edge, tasks of equal probe counts); a large one is planned by CTA 0
-//    behind one more barrier.  Tasks are taken from a counter.
-//  * A task walks its share of the pivot's mids (bt::walk_range): anchor row
-//    in a shared hash or its hub table, each (mid, anchor) pair intersected
-//    from the shorter side, hits queued in shared memory and ruled on in a
-//    dense pass; decrements of the pivot-side and anchor-side edges are summed
-//    in shared memory and flushed once.
+//    crosses hi appends the edge to near.  The next level is known before the
+//    scan: every support that is written or scanned above the level takes part
+//    in a running minimum (see Control::cand), so a level costs one scan and
+//    one barrier.
 //  * Processed edges are dropped from the rows (device-side compaction)
 //    whenever the live edges have halved (the reference's trigger, :537-549,
 //    without its floor at a tenth of the edges); compaction only changes
 //    work, not results.
+// 512 threads a CTA: with 1,024 (64 registers) the lone sub-rounds took 20%
+// longer and only hub rows of 500k edges and more gained (3%).
 // Grid barriers are bounded by a time limit; an expired wait sets an error and
 // the kernel returns.
 #include <cstdio>
@@ -58,67 +82,83 @@
 namespace {
 
 using bt::kEmpty;
-using bt::kThreads;
-constexpr uint32_t kLocalPlan = kMspLocalPlan;  // largest frontier every CTA may plan itself
+constexpr int kThreads = 512;
+constexpr uint32_t kWarps = kThreads / 32;
+constexpr uint32_t kEdges = kMspLocalPlan;  // frontier edges a CTA plans at once
+
+// What every CTA reads after a barrier, in one warp-wide load (barrier()).
+struct Control {
+    unsigned long long delta;      // width of the near bucket
+    unsigned long long far_min;
+    // cand[k % 3]: a lower bound of the supports that are live above level
+    // number k, collected while that level is scanned and peeled
+    unsigned long long cand[3];
+    uint32_t len[3];               // frontier list lengths by sub-round index mod 3
+    uint32_t near_ctr[2];          // near bucket lengths (selector kept by every CTA)
+    uint32_t far_len, far2_len, pad;
+};
+constexpr uint32_t kControlWords = sizeof(Control) / 4;
+static_assert(kControlWords <= 32, "the control words are loaded by one warp");
 
 struct MspState {
     bt::Barrier bar;
-    // control
-    unsigned long long hi, delta;
-    unsigned long long min_sup, far_min;
-    long long edge_num;            // unprocessed edges
-    unsigned long long live_at_compress;
+    __align__(128) Control ctl;
+    // the first entries of the two frontier lists as (edge, U end, V end, 0):
+    // what a short frontier's plan needs, written by whoever appends
+    uint4 head[2][32];
+    uint32_t task_ctr[3];          // chunk counters by sub-round index mod 3
     unsigned long long last_level; // last level with a non-empty frontier
-    uint32_t len[3];               // frontier list lengths by sub-round index mod 3
-    uint32_t task_ctr[3];          // task counters by sub-round index mod 3
-    uint32_t near_ctr[2];          // near bucket lengths (selector kept by every CTA)
-    uint32_t far_len, far2_len;
-    uint32_t task_total, done, overflow;
-    unsigned long long ph_ns[4];   // CTA 0's time in: level transitions, sub-rounds
+    uint32_t pool_used;            // row table buckets given out
+    uint32_t done, overflow;
+    unsigned long long ph_ns[2];   // CTA 0's time in: level transitions, sub-rounds
     unsigned long long prof[8];    // SM cycles summed over CTAs, by step (bt::PF_*)
     // statistics
     unsigned long long subrounds, compressions, tasks, levels_seen, rebuilds;
     // work counters (algorithmic bytes): tasks, row positions walked, anchor
     // slots of the peeled edges, butterflies found, decrements
-    unsigned long long w_mids, w_probes, w_anchor, w_hits, w_decs;
+    unsigned long long w_tasks, w_probes, w_anchor, w_hits, w_decs;
 };
 
+// Counters of one thread.
 struct Work {
-    unsigned long long mids = 0, probes = 0, hits = 0, decs = 0;
+    uint32_t probes = 0, hits = 0, decs = 0;
 };
 
 // Optional per-sub-round trace (BT_MSP_TRACE=<path>): what bounds a sub-round.
 struct TraceRow {
     unsigned long long t_ns;        // sub-round duration seen by CTA 0 (plan to barrier exit)
-    unsigned long long max_task_ns; // longest task
+    unsigned long long max_task_ns; // longest CTA
     unsigned long long walked;      // row positions walked
     uint32_t frontier, tasks;
+};
+
+// Per vertex, one 16-byte load: row start, live degree, first bucket of its
+// row table, and the row's position total (sum of its neighbours' degrees).
+struct __align__(16) VRec {
+    uint32_t off, deg, tab, hop;
 };
 
 struct MspArgs {
     MspState *s;
     uint32_t n, nblocks, exact;
-    uint32_t min_grain, tasks_per_cta, local_plan;  // task schedule (results do not depend on it)
+    uint32_t chunks_per_cta, local_plan;  // schedule, with inv_task (results do not depend on it)
     // row compaction trigger: compact when the live edges fall to cfrac of
     // the live edges at the last compaction, while those were at least
     // cfloor * m (compaction changes work, never results)
     float cfrac, cfloor;
+    float inv_task;                 // 1 / positions of a task
     uint64_t m;
     unsigned long long wait_ns;
-    const uint32_t *off;
     const uint2 *ends;
-    uint32_t *deg, *nbr, *eid;      // live rows (compacted in place)
-    uint32_t *two_hop;              // per vertex: sum of live neighbour degrees (row probe total)
-    uint32_t *rowpre;               // per slot: prefix of the row's neighbour degrees
+    VRec *vrec;
+    uint32_t *nbr, *eid;            // live rows (compacted in place)
+    uint4 *pool;                    // row tables (bt::row_lookup)
     unsigned long long *sup;        // working supports (64-bit)
     uint32_t *sup32;                // working supports when every support fits 32 bits (else null)
     uint32_t *enter;                // sub-round index at which the edge joined a frontier
     uint32_t *result;               // bitruss number per edge
-    uint32_t *list[3];              // frontier lists by sub-round index mod 3
+    uint32_t *list0, *list1;        // frontier lists by sub-round index mod 2
     uint32_t *near_a, *near_b, *far_a, *far_b;
-    uint32_t *pl_piv, *pl_anc, *pl_grain, *pl_total, *task_start;  // plan of a large frontier
-    const uint32_t *hub_base, *hub_mask;
-    const uint2 *hub_pool;
     TraceRow *trace;                // optional, trace_cap rows
     uint32_t trace_cap;
 };
@@ -126,6 +166,8 @@ struct MspArgs {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t next3(uint32_t i) { return i == 2 ? 0 : i + 1; }
 
 __device__ __forceinline__ bool is_done(uint32_t en, uint32_t r) { return en != 0 && en < r; }
 
@@ -137,50 +179,56 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
     return v;
 }
 
-// the peel rule for one butterfly seen from frontier edge uv; returns a 3-bit
-// mask of the edges to decrement: bit0 wv, bit1 wx, bit2 ux
-__device__ __forceinline__ uint32_t peel_rule(uint32_t uv, uint32_t wv, uint32_t wx, uint32_t ux,
-                                              bool cwv, bool cwx, bool cux, uint32_t exact) {
-    const bool pwv = !cwv, pwx = !cwx, pux = !cux;
-    const int cnt = (int)pwv + (int)pwx + (int)pux;
-    uint32_t d = 0;
-    if (cnt == 3) {
-        d = 7;  // peel_three_edge, bitruss_msp.cu:178-184
-    } else if (cnt == 2) {  // peel_two_edge, :148-175
-        if (pwv && pwx && uv < ux) d = 3;
-        if (pwv && pux && uv < wx) d = 5;
-        if (pwx && pux && uv < wv) d = 6;
-    } else if (cnt == 1) {  // peel_one_edge, :126-145
-        if (!exact) {
-            if (pwx && uv < ux && ux < wv) d = 2;
-            if (pwv && uv < ux && ux < wx) d = 1;
-            if (pux && uv < wv && wv < wx) d = 4;
-        } else {  // decrement the survivor once: by the smallest frontier edge
-            if (pwx && uv < ux && uv < wv) d = 2;
-            if (pwv && uv < ux && uv < wx) d = 1;
-            if (pux && uv < wv && uv < wx) d = 4;
-        }
-    }
-    return d;
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-// One sub-round's view of the state.
-struct Round {
-    uint32_t r;                     // sub-round index
-    unsigned long long L, hi;       // level and near-bucket bound
-    uint32_t *next, *next_len;      // next frontier
-    uint32_t *near_list, *near_len;
-};
+__device__ __forceinline__ VRec load_vrec(const VRec *p) {
+    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(p));
+    return VRec{q.x, q.y, q.z, q.w};
+}
 
-// The kernel is compiled twice: N32 = every working support fits 32 bits
-// (4-byte supports and atomics), else 64-bit supports.
+// The peel rule for one butterfly seen from frontier edge uv; returns a 3-bit
+// mask of the edges to decrement: bit0 wv, bit1 wx, bit2 ux.  An edge that is
+// in the frontier itself (c..) is never decremented, and the frontier edges of
+// the butterfly share the work by their ids:
+//  * none besides uv: all three lose one (peel_three_edge, bitruss_msp.cu:178-184);
+//  * one besides uv: the smaller of the two decrements (peel_two_edge, :148-175);
+//  * two besides uv (peel_one_edge, :126-145): exact: the smallest of the three
+//    decrements the survivor.  Reference: with the survivor wv, wx or ux, uv
+//    decrements it only if uv < ux < wx, uv < ux < wv or uv < wv < wx.
+// So uv decrements when its id is below every other frontier edge's, and the
+// reference's rule asks for the order of the other two as well.  Written
+// without branches: lanes of a warp disagree about the case.
+__device__ __forceinline__ uint32_t peel_rule(uint32_t uv, uint32_t wv, uint32_t wx, uint32_t ux, bool cwv,
+                                              bool cwx, bool cux, uint32_t exact) {
+    const uint32_t live = (cwv ? 0u : 1u) | (cwx ? 0u : 2u) | (cux ? 0u : 4u);
+    const bool first = (!cwv | (uv < wv)) & (!cwx | (uv < wx)) & (!cux | (uv < ux));
+    const bool chain = (live == 2 & (ux < wv)) | (live == 1 & (ux < wx)) | (live == 4 & (wv < wx));
+    const bool one = live == 1 | live == 2 | live == 4;
+    return first & (!one | (exact != 0) | chain) ? live : 0u;
+}
+
+// The kernel is compiled twice: N32 = every working support is below 2^32 - 1
+// (4-byte supports, levels and atomics), else 64-bit supports.
 template <bool N32>
 using SupWord = typename std::conditional<N32, uint32_t, unsigned long long>::type;
 
+// One sub-round's view of the state.
 template <bool N32>
-__device__ __forceinline__ unsigned long long sup_of(const MspArgs &a, uint32_t e) {
-    if constexpr (N32) return a.sup32[e];
-    else return a.sup[e];
+struct Round {
+    uint32_t r;                     // sub-round index
+    SupWord<N32> L, hi;             // level and near-bucket bound
+    uint32_t *next, *next_len;      // next frontier
+    uint4 *next_head;
+    uint32_t *near_list, *near_len;
+};
+
+template <bool N32>
+__device__ __forceinline__ SupWord<N32> sup_of(const MspArgs &a, uint32_t e) {
+    if constexpr (N32) return __ldcg(a.sup32 + e);
+    else return __ldcg(a.sup + e);
 }
 
 // Subtract k from sup[e].  The decrement that takes it from above L to L or
@@ -199,270 +247,359 @@ __device__ __forceinline__ SupWord<N32> dec_issue(const MspArgs &a, uint32_t e, 
     else return atomicAdd(a.sup + e, (unsigned long long)(-(long long)k));
 }
 
-__device__ __forceinline__ void dec_settle(const MspArgs &a, const Round &rd, uint32_t e, uint32_t k,
-                                           unsigned long long old) {
-    const unsigned long long nw = old - k;
-    if (old > rd.L && nw <= rd.L) {
-        rd.next[atomicAdd(rd.next_len, 1u)] = e;
-        a.enter[e] = rd.r + 1;
-        a.result[e] = (uint32_t)rd.L;
+// Append n of the edges e[0..2] (those in `mask`) to a frontier list.
+__device__ __forceinline__ void list_append(const MspArgs &a, uint32_t *list, uint32_t *len, uint4 *head,
+                                            uint32_t e0, uint32_t e1, uint32_t e2, uint32_t mask, uint32_t stamp,
+                                         uint32_t value) {
+    const uint32_t e[3] = {e0, e1, e2};
+    uint2 ends[3];
+#pragma unroll
+    for (uint32_t q = 0; q < 3; q++)
+        if (mask >> q & 1) ends[q] = __ldg(a.ends + e[q]);  // beside the counter's round trip
+    uint32_t at = atomicAdd(len, (uint32_t)__popc(mask));
+#pragma unroll
+    for (uint32_t q = 0; q < 3; q++)
+        if (mask >> q & 1) {
+            list[at] = e[q];
+            if (at < 32) head[at] = make_uint4(e[q], ends[q].x, ends[q].y, 0);
+            at++;
+            a.enter[e[q]] = stamp;
+            a.result[e[q]] = value;
+        }
+}
+
+// Settle up to three decrements, of k[q] on e[q] with old support old[q] (0:
+// none).  low: the thread's running minimum of the supports left above the
+// level.
+template <bool N32>
+__device__ __forceinline__ void dec_settle(const MspArgs &a, const Round<N32> &rd, const uint32_t (&e)[3],
+                                           uint32_t k2, const SupWord<N32> (&old)[3], SupWord<N32> &low) {
+    uint32_t push = 0, near = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 3; q++) {
+        const SupWord<N32> nw = old[q] - (q == 2 ? k2 : 1u);
+        if (old[q] > rd.L) {
+            if (nw > rd.L) low = nw < low ? nw : low;
+            else push |= 1u << q;
+            if (old[q] >= rd.hi && nw < rd.hi) near |= 1u << q;
+        }
     }
-    if (old >= rd.hi && nw < rd.hi) rd.near_list[atomicAdd(rd.near_len, 1u)] = e;
+    if (push) list_append(a, rd.next, rd.next_len, rd.next_head, e[0], e[1], e[2], push, rd.r + 1, (uint32_t)rd.L);
+    if (near) {
+        uint32_t at = atomicAdd(rd.near_len, (uint32_t)__popc(near));
+#pragma unroll
+        for (uint32_t q = 0; q < 3; q++)
+            if (near >> q & 1) rd.near_list[at++] = e[q];
+    }
 }
 
 // ---------------------------------------------------------------------------
 // shared memory
 // ---------------------------------------------------------------------------
 
+// Frontier edges as this CTA has planned them.
 struct Smem {
-    bt::Walk walk;
-    // plan of a small frontier (every CTA computes it)
-    uint32_t lp_piv[kLocalPlan];
-    uint32_t lp_anc[kLocalPlan];
-    uint32_t lp_grain[kLocalPlan];
-    uint32_t lp_total[kLocalPlan];
-    uint32_t lp_start[kLocalPlan + 1];
-    uint32_t task, idx;
-    uint32_t running;
-    unsigned long long total;
+    uint32_t e_uv[kEdges], e_piv[kEdges], e_anc[kEdges];
+    uint32_t e_po[kEdges], e_pd[kEdges];   // pivot row: start, degree
+    uint32_t e_ao[kEdges], e_ad[kEdges], e_at[kEdges];  // anchor row: start, degree, table
+    uint32_t e_info[kEdges];               // log2 of the tasks that share a block of mids; kPivIsV
+    uint32_t e_pre[kEdges + 1];            // exclusive prefix of the task counts
+    uint32_t dec[kThreads];                // per warp and mid: pending pivot-side decrements
+    uint32_t wsum[kWarps];
+    unsigned long long low;                // running minimum of the supports above the level
+    uint32_t chunk, total, next_task;
+    Control now;                           // the control words as of the last barrier
+    unsigned long long tasks, anchor;      // counters of this CTA
+    unsigned long long prof_t, prof[8];    // see bt::PF_*
 };
 
-__device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm) {
-    bt::prof_mark(sm.walk, bt::PF_OTHER);
-    const bool ok = bt::grid_barrier(&a.s->bar, a.nblocks, a.wait_ns);
-    bt::prof_mark(sm.walk, bt::PF_BARRIER);
-    return ok;
+constexpr uint32_t kPivIsV = 0x80000000u;  // the pivot is the edge's V end
+
+// Time accounting and bookkeeping are done by a CTA's last thread: the first
+// warp plans and has the first task, so it is on the longest path.
+__device__ __forceinline__ bool is_clerk() { return threadIdx.x == kThreads - 1; }
+
+__device__ __forceinline__ void prof_mark(Smem &sm, int k) {
+    if (is_clerk()) {
+        const unsigned long long t = clock64();
+        sm.prof[k] += t - sm.prof_t;
+        sm.prof_t = t;
+    }
+}
+
+// The control words and the head of a frontier list (lane i: entry i), by the
+// first warp (the caller synchronises the block).
+// One request per CTA: the same word read by all 2,432 warps of the grid at
+// once is served one request at a time by its L2 slice (about a microsecond).
+__device__ __forceinline__ uint4 load_control(const MspArgs &a, Smem &sm, uint32_t list) {
+    const uint4 head = __ldcg(&a.s->head[list][threadIdx.x]);
+    if (threadIdx.x < kControlWords)
+        reinterpret_cast<uint32_t *>(&sm.now)[threadIdx.x] =
+            __ldcg(reinterpret_cast<const uint32_t *>(&a.s->ctl) + threadIdx.x);
+    return head;
 }
 
 // ---------------------------------------------------------------------------
-// plan: orientation of every frontier edge and tasks of equal probe counts
-// ---------------------------------------------------------------------------
-//
-// The pivot is the endpoint whose row's probe total (two_hop) is smaller.  The
-// grain is the sub-round's total over tasks_per_cta tasks per CTA (tasks are
-// taken dynamically, so a few per CTA even out their unequal real costs), at
-// least min_grain and, for an anchor staged in shared memory, at least twice
-// its row (each task stages that row).
-// Writes piv/anc per edge, the grain (bit 31: the pivot is the V end), the
-// pivot row's probe total and the exclusive prefix of task counts
-// (start[len] = number of tasks).  Runs on one whole CTA.
-constexpr uint32_t kPivIsV = 0x80000000u;
-__device__ void plan(const MspArgs &a, Smem &sm, const uint32_t *curr, uint32_t len, uint32_t *piv_out,
-                     uint32_t *anc_out, uint32_t *grain_out, uint32_t *total_out, uint32_t *start_out,
-                     bool count_anchor) {
-    if (threadIdx.x == 0) {
-        sm.running = 0;
-        sm.total = 0;
-    }
-    __syncthreads();
-    unsigned long long mine = 0;
-    for (uint32_t i = threadIdx.x; i < len; i += kThreads) {
-        const uint32_t e = curr[i];
-        const uint2 uv = a.ends[e];
-        const uint32_t cu = a.two_hop[uv.x], cv = a.two_hop[uv.y];
-        piv_out[i] = cv <= cu ? uv.y : uv.x;
-        anc_out[i] = cv <= cu ? uv.x : uv.y;
-        total_out[i] = cv <= cu ? cv : cu;
-        grain_out[i] = cv <= cu ? kPivIsV : 0;
-        mine += cv <= cu ? cv : cu;
-    }
-    for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&sm.total, mine);
-    __syncthreads();
-    unsigned long long g = sm.total / ((unsigned long long)a.tasks_per_cta * a.nblocks);
-    if (g < a.min_grain) g = a.min_grain;
-    if (g > (1u << 30)) g = 1u << 30;
-    unsigned long long anchor = 0;
-    for (uint32_t base = 0; base < len; base += kThreads) {
-        const uint32_t i = base + threadIdx.x;
-        uint32_t nt = 0;
-        if (i < len) {
-            const uint32_t anc = anc_out[i];
-            const uint32_t work = total_out[i];
-            const uint32_t da = a.deg[anc];
-            // a task stages a short anchor row in shared memory: make it worth it
-            unsigned long long gi = (da <= bt::kHashMaxDeg && 2ull * da > g) ? 2ull * da : g;
-            if (gi > (1u << 30)) gi = 1u << 30;  // leaves bit 31 for kPivIsV
-            nt = (uint32_t)((work + gi - 1) / gi);
-            grain_out[i] |= (uint32_t)gi;
-            anchor += da;
-        }
-        uint32_t excl, tot;
-        cub::BlockScan<uint32_t, kThreads>(sm.walk.scan).ExclusiveSum(nt, excl, tot);
-        if (i < len) start_out[i] = sm.running + excl;
-        __syncthreads();
-        if (threadIdx.x == 0) sm.running += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) start_out[len] = sm.running;
-    if (count_anchor) {
-        for (int o = 16; o; o >>= 1) anchor += __shfl_xor_sync(0xffffffffu, anchor, o);
-        if ((threadIdx.x & 31) == 0 && anchor) atomicAdd(&a.s->w_anchor, anchor);
-    }
-    __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// peel: all tasks of one sub-round
+// peel
 // ---------------------------------------------------------------------------
 
-// The rule applied to the butterflies of one frontier edge uv (see
-// bt::walk_range for the two-step interface).
-template <bool N32>
-struct MspHit {
-    const MspArgs &a;
-    bt::Walk &w;
-    const Round &rd;
-    uint32_t uv, exact;
-    bool piv_is_v;
-    unsigned long long decs = 0, hits = 0;
-    struct State {
-        uint32_t kslot, e_my, e_ay, ah;
-        // After load(): the stamps of e_my and e_ay.  After apply(): the old
-        // supports of the global decrements the hit has in flight, 0 for none
-        // (a decremented edge's old support is at least 1: an edge loses at
-        // most one support per butterfly it is in).  One pair of fields for
-        // both keeps a lane's four hits within the register budget.
-        SupWord<N32> x_my, x_ay;
-    };
-    __device__ __forceinline__ void load(State &s, uint32_t kk, uint32_t e_my, uint32_t ah) const {
-        s.kslot = kk & ~(uint32_t)bt::kRevHit;
-        s.e_my = e_my;
-        s.ah = ah;
-        s.e_ay = bt::walk_anchor_edge(w, ah);
-        s.x_my = a.enter[e_my];
-        s.x_ay = a.enter[s.e_ay];
-    }
-    // The rule for one hit.  Pivot-side and staged anchor-side decrements are
-    // summed in shared memory; the others are issued here and settled by
-    // settle() once every hit of the lane has issued its own.
-    __device__ __forceinline__ void apply(State &s) {
-        const uint32_t r = rd.r;
-        hits++;  // a butterfly visited (the reference's intersection hit)
-        const uint32_t en_my = (uint32_t)s.x_my, en_ay = (uint32_t)s.x_ay;
-        s.x_my = s.x_ay = 0;
-        if (is_done(en_ay, r) || is_done(en_my, r)) return;
-        const uint32_t e_pm = w.mid_eid[s.kslot];
-        const bool c_pm = w.pm_curr[s.kslot], c_my = en_my == r, c_ay = en_ay == r;
-        // name the edges as the reference does: w on u's side, x on v's
-        uint32_t wv, ux;
-        bool cwv, cux;
-        if (piv_is_v) { wv = e_pm; ux = s.e_ay; cwv = c_pm; cux = c_ay; }
-        else { wv = s.e_ay; ux = e_pm; cwv = c_ay; cux = c_pm; }
-        const uint32_t d = peel_rule(uv, wv, s.e_my, ux, cwv, c_my, cux, exact);
-        if (!d) return;
-        const bool d_wv = d & 1, d_wx = d & 2, d_ux = d & 4;
-        const bool dec_pm = piv_is_v ? d_wv : d_ux;
-        const bool dec_ay = piv_is_v ? d_ux : d_wv;
-        decs += (uint32_t)dec_pm + (uint32_t)d_wx + (uint32_t)dec_ay;
-        if (dec_pm) atomicAdd(&w.slot_dec[s.kslot], 1u);
-        if (d_wx) s.x_my = dec_issue<N32>(a, s.e_my, 1);
-        if (dec_ay) {
-            if (w.cached_size) atomicAdd(&w.hdec[s.ah], 1u);
-            else s.x_ay = dec_issue<N32>(a, s.e_ay, 1);
-        }
-    }
-    __device__ __forceinline__ void settle(const State &s) const {
-        if (s.x_my) dec_settle(a, rd, s.e_my, 1, s.x_my);
-        if (s.x_ay) dec_settle(a, rd, s.e_ay, 1, s.x_ay);
-    }
-    __device__ __forceinline__ void stretch_done() const {}
-    __device__ __forceinline__ bool stop() const { return false; }  // a peel walks every butterfly
-};
-
-template <bool N32>
-__device__ void peel_tasks(const MspArgs &a, Smem &sm, const uint32_t *curr, uint32_t curr_len,
-                           const uint32_t *pl_piv, const uint32_t *pl_anc, const uint32_t *pl_grain,
-                           const uint32_t *pl_total, const uint32_t *start, uint32_t ntasks, uint32_t *ctr,
-                           const Round &rd, uint32_t epoch, Work &wk) {
-    const bt::Rows rows{a.off, a.deg, a.nbr, a.eid, a.hub_base, a.hub_mask, a.hub_pool};
-    const uint32_t *enter = a.enter;
-    const uint32_t r = rd.r;
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
     const uint32_t lane = threadIdx.x & 31;
-    bt::Walk &w = sm.walk;
-    bool first = true;
-    for (;;) {
-        if (threadIdx.x < 32) {
-            // the first task of every CTA is its block index; the rest come
-            // from the counter, which starts at the number of CTAs
-            uint32_t t = blockIdx.x;
-            if (!first && lane == 0) t = gridDim.x + atomicAdd(ctr, 1u);
-            t = __shfl_sync(0xffffffffu, t, 0);
-            uint32_t i = 0;
-            if (t < ntasks) i = bt::warp_find_slot(start, curr_len, t);  // last i: start[i] <= t
-            if (lane == 0) {
-                sm.task = t;
-                sm.idx = i;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += t;
+    }
+    return v;
+}
+
+// Plan frontier edge e as entry i: orientation and tasks; returns their number.
+//  * The pivot is the endpoint whose row's position total is smaller; both
+//    orientations visit the same butterflies.
+//  * A task is a warp on a block of 32 of the pivot's mids, or, where their
+//    rows hold more positions than a task should (1 / inv_task), on an equal
+//    part of them: a power of two of parts, at most about `budget` tasks for
+//    the edge, beyond which the warps of the grid have enough to do.
+__device__ __forceinline__ uint32_t plan_edge(const MspArgs &a, Smem &sm, uint32_t i, uint32_t e, uint2 uv,
+                                              float budget, uint32_t &anchor) {
+    const VRec ru = load_vrec(a.vrec + uv.x), rv = load_vrec(a.vrec + uv.y);
+    const bool pv = rv.hop <= ru.hop;
+    const VRec &p = pv ? rv : ru, &q = pv ? ru : rv;
+    const uint32_t blocks = (p.deg + 31) >> 5;
+    // positions of a block: every mid has at most the anchor's degree
+    const float est = fminf((float)p.hop, (float)p.deg * (float)q.deg);
+    const float parts = __fdividef(fminf(est * a.inv_task, budget), (float)blocks);
+    const int lg = parts > 1.0f ? min(16, (__float_as_int(parts) >> 23) - 126) : 0;  // ceil(log2), or one more
+    sm.e_uv[i] = e;
+    sm.e_piv[i] = pv ? uv.y : uv.x;
+    sm.e_anc[i] = pv ? uv.x : uv.y;
+    sm.e_po[i] = p.off;
+    sm.e_pd[i] = p.deg;
+    sm.e_ao[i] = q.off;
+    sm.e_ad[i] = q.deg;
+    sm.e_at[i] = q.tab;
+    sm.e_info[i] = (uint32_t)lg | (pv ? kPivIsV : 0u);
+    anchor = q.deg;
+    return blocks << lg;
+}
+
+// Plan up to 32 edges (lane i: entry h of frontier edge i) by one warp; the
+// caller synchronises the block.
+__device__ __forceinline__ void plan_warp(const MspArgs &a, Smem &sm, uint32_t cnt, uint4 h, uint32_t warps,
+                                          bool count_anchor) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t t = 0, anchor = 0;
+    if (lane < cnt)
+        t = plan_edge(a, sm, lane, h.x, make_uint2(h.y, h.z), __fdividef(4.0f * (float)warps, (float)cnt) + 1.0f,
+                      anchor);
+    const uint32_t inc = warp_inclusive(t);
+    if (lane < cnt) sm.e_pre[lane] = inc - t;
+    if (lane == 31) {
+        sm.total = inc;
+        sm.next_task = kWarps;
+    }
+    if (count_anchor) {
+        anchor = __reduce_add_sync(0xffffffffu, anchor);
+        if (lane == 0) sm.anchor += anchor;
+    }
+}
+
+// Plan curr[0, cnt) (cnt <= kEdges) for `warps` warps.  Ends synchronised.
+__device__ __forceinline__ void plan_block(const MspArgs &a, Smem &sm, const uint32_t *curr, uint32_t cnt,
+                                           uint32_t warps, bool count_anchor) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = threadIdx.x;
+    uint32_t t = 0, anchor = 0;
+    if (i < cnt) {
+        const uint32_t e = __ldcg(curr + i);
+        t = plan_edge(a, sm, i, e, __ldg(a.ends + e), __fdividef(4.0f * (float)warps, (float)cnt) + 1.0f, anchor);
+    }
+    const uint32_t inc = warp_inclusive(t);
+    if (lane == 31) sm.wsum[warp] = inc;
+    anchor = __reduce_add_sync(0xffffffffu, anchor);
+    if (lane == 0 && count_anchor) atomicAdd(&sm.anchor, (unsigned long long)anchor);
+    __syncthreads();
+    const uint32_t w = warp_inclusive(lane < kWarps ? sm.wsum[lane] : 0);
+    const uint32_t before = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0);
+    if (i < cnt) sm.e_pre[i] = (warp ? before : 0) + inc - t;
+    if (i == kThreads - 1) {
+        sm.total = (warp ? before : 0) + inc;
+        sm.next_task = kWarps;
+    }
+    __syncthreads();
+}
+
+// Grid barrier.  Publishes the CTA's running minimum to cand[k3], refreshes
+// sm.now, and with `plan` plans the next frontier (length len[r3], list `list`)
+// when it is a short one: its entries come with the control words.
+__device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm, uint32_t &epoch, uint32_t k3, uint32_t r3,
+                                        uint32_t list, bool plan) {
+    __syncthreads();
+    prof_mark(sm, bt::PF_OTHER);
+    int ok = 1;
+    if (threadIdx.x < 32) {
+        const unsigned long long low = sm.low;
+        __syncwarp();
+        if (threadIdx.x == 0) {
+            // (sm.now is of the last barrier: cand only falls meanwhile)
+            if (low < sm.now.cand[k3]) atomicMin(&a.s->ctl.cand[k3], low);
+            sm.low = ~0ull;
+        }
+        __syncwarp();
+        epoch += a.nblocks;
+        ok = bt::barrier_wait(&a.s->bar, epoch, a.wait_ns);
+        const uint4 head = load_control(a, sm, list);
+        __syncwarp();
+        const uint32_t len = sm.now.len[r3];
+        if (plan && len - 1 < 32 && len <= a.local_plan)
+            plan_warp(a, sm, len, head, a.nblocks * kWarps, blockIdx.x == 0);
+    }
+    ok = __syncthreads_and(ok);
+    prof_mark(sm, bt::PF_BARRIER);
+    return ok != 0;
+}
+
+// Every thread's running minimum into the CTA's (before a barrier).
+template <bool N32>
+__device__ __forceinline__ void fold_low(Smem &sm, SupWord<N32> low) {
+    if constexpr (N32) low = __reduce_min_sync(0xffffffffu, low);
+    else low = warp_min(low);
+    if ((threadIdx.x & 31) == 0 && low != (SupWord<N32>)~0ull) atomicMin(&sm.low, (unsigned long long)low);
+}
+
+constexpr uint32_t kRev = 0x40000000u;     // the anchor's row is walked, the mid's table looked up
+constexpr uint32_t kPmCurr = 0x80000000u;  // edge (pivot, mid) is in the frontier
+constexpr uint32_t kNbMask = 0x3fffffffu;
+
+// Run this CTA's tasks (first + step * j for j = 0, 1, ..., below `tasks`) of
+// the planned edges and rule on every butterfly found.  Its warps take them
+// one by one; no block barriers.
+template <bool N32>
+__device__ __forceinline__ void run_tasks(const MspArgs &a, Smem &sm, uint32_t cnt, uint32_t tasks, uint32_t first,
+                                          uint32_t step, const Round<N32> &rd, Work &wk, SupWord<N32> &low) {
+    const uint32_t lane = threadIdx.x & 31, r = rd.r;
+    uint32_t *dec = sm.dec + (threadIdx.x & ~31u);
+    for (uint32_t task = first + step * (threadIdx.x >> 5); task < tasks;) {
+        const uint32_t i = bt::warp_find_slot(sm.e_pre, cnt, task);
+        const uint32_t lg = sm.e_info[i] & 31, piv = sm.e_piv[i], ad = sm.e_ad[i];
+        const uint32_t local = task - sm.e_pre[i], part = local & ((1u << lg) - 1);
+        // one mid per lane: shorter side, table and length of the (mid, anchor) pair
+        const uint32_t k = (local >> lg) * 32 + lane;
+        uint32_t row = 0, tab = 0, nb = 0, e_pm = 0, len = 0;
+        if (k < sm.e_pd[i]) {
+            const uint32_t pos = sm.e_po[i] + k;
+            const uint32_t mid = a.nbr[pos];
+            e_pm = a.eid[pos];
+            const uint32_t en = a.enter[e_pm];
+            const VRec rm = load_vrec(a.vrec + mid);
+            if (mid != sm.e_anc[i] && !is_done(en, r)) {
+                const bool rev = ad < rm.deg;
+                row = rev ? sm.e_ao[i] : rm.off;
+                tab = rev ? rm.tab : sm.e_at[i];
+                nb = bt_row_buckets(rev ? rm.deg : ad) | (rev ? kRev : 0u) | (en == r ? kPmCurr : 0u);
+                len = rev ? ad : rm.deg;
             }
         }
-        __syncthreads();
-        first = false;
-        const uint32_t t = sm.task;
-        if (t >= ntasks) break;
-        const unsigned long long task_t0 = (a.trace && threadIdx.x == 0) ? bt::global_ns() : 0;
-        const unsigned long long walked0 = w.walked;
-        const uint32_t i = sm.idx, k = t - start[i];
-        const uint32_t uv = curr[i];
-        const uint32_t piv = pl_piv[i], anc = pl_anc[i], gword = pl_grain[i];
-        const uint32_t gi = gword & ~kPivIsV, total = pl_total[i];
-        const bool piv_is_v = (gword & kPivIsV) != 0;
-        const uint32_t f0 = k * gi;
-        const uint32_t f1 = total - f0 < gi ? total : f0 + gi;
-        const uint32_t exact = a.exact;
-        if (threadIdx.x == 0) wk.mids++;
-        bt::prof_mark(w, bt::PF_TASK);
-        MspHit<N32> hit{a, w, rd, uv, exact, piv_is_v};
-        bt::walk_range(
-            rows, a.rowpre, w, piv, anc, epoch, total, f0, f1,
-            [&](uint32_t kk, uint32_t e_pm) {
-                const uint32_t en = enter[e_pm];
-                w.pm_curr[kk] = en == r;
-                return !is_done(en, r);
-            },
-            hit,
-            [&](uint32_t cl, bool last) {
-                // flush the pivot-side decrements of the slice and, after the
-                // last slice, the anchor-side decrements of the task
-                // (every decrement of a thread is issued before any is settled)
-                __syncthreads();
-                uint32_t c = 0;
-                SupWord<N32> old = 0;
-                if (threadIdx.x < cl) {
-                    c = w.slot_dec[threadIdx.x];
-                    if (c) {
-                        w.slot_dec[threadIdx.x] = 0;
-                        old = dec_issue<N32>(a, w.mid_eid[threadIdx.x], c);
-                    }
-                }
-                constexpr uint32_t kPer = bt::kHashSlots / kThreads;
-                uint32_t hc[kPer];
-                SupWord<N32> hold[kPer];
-                const uint32_t hsize = last ? w.cached_size : 0;
-#pragma unroll
-                for (uint32_t q = 0; q < kPer; q++) {
-                    const uint32_t h = threadIdx.x + q * kThreads;
-                    hc[q] = 0;
-                    hold[q] = 0;
-                    if (h < hsize) {
-                        hc[q] = w.hdec[h];
-                        if (hc[q]) {
-                            w.hdec[h] = 0;
-                            hold[q] = dec_issue<N32>(a, w.hval[h], hc[q]);
-                        }
-                    }
-                }
-                if (c) dec_settle(a, rd, w.mid_eid[threadIdx.x], c, old);
-#pragma unroll
-                for (uint32_t q = 0; q < kPer; q++)
-                    if (hc[q]) dec_settle(a, rd, w.hval[threadIdx.x + q * kThreads], hc[q], hold[q]);
-            });
-        wk.decs += hit.decs;
-        wk.hits += hit.hits;
-        bt::prof_mark(w, bt::PF_FLUSH);
-        if (a.trace && threadIdx.x == 0 && r < a.trace_cap) {
-            atomicMax(&a.trace[r].max_task_ns, bt::global_ns() - task_t0);
-            atomicAdd(&a.trace[r].walked, w.walked - walked0);
+        uint32_t pre = warp_inclusive(len);
+        const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
+        pre -= len;
+        // this part's positions: [total * part / 2^lg, total * (part + 1) / 2^lg)
+        uint32_t f0 = 0, f1 = total;
+        if (lg) {
+            const uint32_t q = total >> lg, rem = total & ((1u << lg) - 1);
+            f0 = q * part + (rem * part >> lg);
+            f1 = q * (part + 1) + (rem * (part + 1) >> lg);
         }
+        if (lane == 0) wk.probes += f1 - f0;
+        // decrements in flight: each is settled a round later, beside that
+        // round's loads, the last ones beside the pivot-side decrement
+        uint32_t pe[3] = {0, 0, e_pm};
+        SupWord<N32> old[3] = {0, 0, 0};
+        for (uint32_t fb = f0; fb < f1; fb += 32) {
+            const uint32_t f = fb + lane;
+            // the mid of position f: the last lane with pre <= f and a position of its own
+            uint32_t m = 0;
+#pragma unroll
+            for (uint32_t o = 16; o; o >>= 1) {
+                const uint32_t t = __shfl_sync(0xffffffffu, pre, m + o);
+                if (t <= f) m += o;
+            }
+            const uint32_t mrow = __shfl_sync(0xffffffffu, row, m), mtab = __shfl_sync(0xffffffffu, tab, m);
+            const uint32_t mnb = __shfl_sync(0xffffffffu, nb, m), mpre = __shfl_sync(0xffffffffu, pre, m);
+            const uint32_t mpm = __shfl_sync(0xffffffffu, e_pm, m);
+            uint32_t y = piv, e1 = 0;
+            if (f < f1) {
+                y = a.nbr[mrow + (f - mpre)];
+                e1 = a.eid[mrow + (f - mpre)];
+            }
+            dec_settle<N32>(a, rd, pe, 0, old, low);
+            old[0] = old[1] = 0;
+            if (y == piv) continue;
+            const bt::RowPlace at = bt::row_place(y, mnb & kNbMask);
+            const bt::RowBucket q1 = bt::row_bucket(a.pool, mtab, at.h1);
+            const bt::RowBucket q2 = bt::row_bucket(a.pool, mtab, at.h2);
+            const uint32_t en1 = a.enter[e1];
+            const uint32_t e2 = bt::row_resolve(a.pool, mtab, mnb & kNbMask, at, q1, q2, y);
+            if (e2 == kEmpty) continue;
+            wk.hits++;  // a butterfly visited (the reference's intersection hit)
+            const uint32_t en2 = a.enter[e2];
+            if (is_done(en1, r) || is_done(en2, r)) continue;
+            const bool rev = mnb & kRev, isv = sm.e_info[i] & kPivIsV;
+            const uint32_t e_my = rev ? e2 : e1, e_ay = rev ? e1 : e2;
+            const bool c1 = en1 == r, c2 = en2 == r, c_pm = mnb & kPmCurr;
+            const bool c_my = rev ? c2 : c1, c_ay = rev ? c1 : c2;
+            // name the edges as the reference does: w on u's side, x on v's
+            const uint32_t d = peel_rule(sm.e_uv[i], isv ? mpm : e_ay, e_my, isv ? e_ay : mpm, isv ? c_pm : c_ay,
+                                         c_my, isv ? c_ay : c_pm, a.exact);
+            wk.decs += __popc(d);
+            const bool d_wv = d & 1, d_wx = d & 2, d_ux = d & 4;
+            const bool d_ay = isv ? d_ux : d_wv;
+            pe[0] = e1;
+            pe[1] = e2;
+            if (rev ? d_ay : d_wx) old[0] = dec_issue<N32>(a, e1, 1);
+            if (rev ? d_wx : d_ay) old[1] = dec_issue<N32>(a, e2, 1);
+            if (isv ? d_wv : d_ux) atomicAdd(dec + m, 1u);
+        }
+        // the next task, and the pivot-side decrements: one edge per mid
+        uint32_t j = 0;
+        if (lane == 0) j = atomicAdd(&sm.next_task, 1u);
+        __syncwarp();
+        const uint32_t n_pm = dec[lane];
+        if (n_pm) {
+            dec[lane] = 0;
+            old[2] = dec_issue<N32>(a, e_pm, n_pm);
+        }
+        dec_settle<N32>(a, rd, pe, n_pm, old, low);
+        __syncwarp();
+        task = first + step * __shfl_sync(0xffffffffu, j, 0);
+    }
+}
+
+// Peel the frontier curr[0, len): one sub-round without its barrier (which
+// has planned it already when it is short).
+template <bool N32>
+__device__ __forceinline__ void peel(const MspArgs &a, Smem &sm, const uint32_t *curr, uint32_t len, uint32_t *ctr,
+                                     const Round<N32> &rd, Work &wk, SupWord<N32> &low) {
+    const uint32_t rank = blockIdx.x, size = a.nblocks;
+    // a frontier that every CTA plans whole, its tasks dealt to all CTAs, or
+    // chunks of it that a CTA plans and runs alone: its first is its own
+    // rank, the rest come from the counter
+    const bool whole = len <= a.local_plan;
+    uint32_t chunk = len;
+    if (!whole) {
+        chunk = len / (size * a.chunks_per_cta) + 1;
+        chunk = chunk < 8 ? 8 : chunk > kEdges ? kEdges : chunk;
+    }
+    for (uint32_t c = whole ? 0 : rank; c * chunk < len;) {
+        const uint32_t first = c * chunk, cnt = len - first < chunk ? len - first : chunk;
+        if (!whole && threadIdx.x == 0) sm.chunk = size + atomicAdd(ctr, 1u);
+        if (!whole || cnt > 32) plan_block(a, sm, curr + first, cnt, whole ? size * kWarps : kWarps, !whole || rank == 0);
+        const uint32_t tasks = sm.total;
+        if (is_clerk() && (!whole || rank == 0)) sm.tasks += tasks;
+        run_tasks<N32>(a, sm, cnt, tasks, whole ? rank : 0, whole ? size : 1, rd, wk, low);
+        if (whole) break;
+        __syncthreads();
+        c = sm.chunk;
+        __syncthreads();
     }
 }
 
@@ -472,15 +609,14 @@ __device__ void peel_tasks(const MspArgs &a, Smem &sm, const uint32_t *curr, uin
 
 // Minimum support over the live entries of `list` (grid-wide atomicMin).
 template <bool N32>
-__device__ void list_min(const MspArgs &a, const uint32_t *list, uint32_t len, unsigned long long *out) {
+__device__ __forceinline__ void list_min(const MspArgs &a, const uint32_t *list, uint32_t len, unsigned long long *out) {
     unsigned long long v = ~0ull;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
     for (uint32_t i = gtid; i < len; i += gsz) {
-        const uint32_t e = list[i];
-        if (a.enter[e] == 0) {
-            const unsigned long long s = sup_of<N32>(a, e);
-            v = s < v ? s : v;
-        }
+        const uint32_t e = __ldcg(list + i);
+        const uint32_t en = __ldcg(a.enter + e);
+        const unsigned long long s = sup_of<N32>(a, e);
+        if (en == 0) v = s < v ? s : v;
     }
     v = warp_min(v);
     if ((threadIdx.x & 31) == 0 && v != ~0ull) atomicMin(out, v);
@@ -488,12 +624,12 @@ __device__ void list_min(const MspArgs &a, const uint32_t *list, uint32_t len, u
 
 // Drop processed edges (enter in (0, r)) from every row; one warp per vertex,
 // in place.
-__device__ void compress_rows(const MspArgs &a, uint32_t r) {
+__device__ __forceinline__ void compress_rows(const MspArgs &a, uint32_t r) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t x = warp; x < a.n; x += nw) {
-        const uint32_t b = a.off[x], d = a.deg[x];
+        const uint32_t b = a.vrec[x].off, d = a.vrec[x].deg;
         uint32_t w = 0;
         for (uint32_t j0 = 0; j0 < d; j0 += 32) {
             const uint32_t j = j0 + lane;
@@ -502,7 +638,7 @@ __device__ void compress_rows(const MspArgs &a, uint32_t r) {
             if (j < d) {
                 y = a.nbr[b + j];
                 e = a.eid[b + j];
-                keep = !is_done(a.enter[e], r);
+                keep = !is_done(__ldcg(a.enter + e), r);
             }
             const uint32_t bal = __ballot_sync(0xffffffffu, keep);
             __syncwarp();
@@ -514,13 +650,24 @@ __device__ void compress_rows(const MspArgs &a, uint32_t r) {
             w += __popc(bal);
             __syncwarp();
         }
-        if (lane == 0) a.deg[x] = w;
+        if (lane == 0) a.vrec[x].deg = w;
     }
 }
 
-__device__ void compute_two_hop(const MspArgs &a) {
-    const bt::Rows rows{a.off, a.deg, a.nbr, a.eid, a.hub_base, a.hub_mask, a.hub_pool};
-    bt::row_prefix(rows, a.n, a.rowpre, a.two_hop);
+// Position total and table of every row; one warp per vertex.
+__device__ __forceinline__ void prepare_rows(const MspArgs &a) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t x = warp; x < a.n; x += nw) {
+        const VRec v = load_vrec(a.vrec + x);
+        if (v.deg == 0) continue;
+        unsigned long long hop = 0;
+        for (uint32_t j = lane; j < v.deg; j += 32) hop += __ldcg(&a.vrec[a.nbr[v.off + j]].deg);
+        hop = warp_sum(hop);
+        if (lane == 0) a.vrec[x].hop = hop > 0xffffffffull ? 0xffffffffu : (uint32_t)hop;
+        bt::row_build(a.pool, v.tab, v.deg, a.nbr + v.off, a.eid + v.off);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -528,178 +675,204 @@ __device__ void compute_two_hop(const MspArgs &a) {
 // ---------------------------------------------------------------------------
 
 template <bool N32>
-__global__ void __launch_bounds__(kThreads, 1) k_msp(MspArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ MspArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     MspState *s = a.s;
-    bt::walk_init(sm.walk);
+    if (threadIdx.x == 0) {
+        sm.low = ~0ull;
+        sm.tasks = sm.anchor = 0;
+        for (int k = 0; k < 8; k++) sm.prof[k] = 0;
+    }
+    if (is_clerk()) sm.prof_t = clock64();
+    if (threadIdx.x < 32) load_control(a, sm, 0);
+    sm.dec[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
-    constexpr uint32_t kNearTarget = 1u << 16;
+    const bool clerk = blockIdx.x == 0 && is_clerk();
     Work wk;
-    uint32_t r = 2;            // sub-round index (1 marks the zero-support edges)
-    uint32_t epoch = 0;        // row compactions so far (same in every CTA)
-    unsigned long long L = 0;  // current level (same in every CTA)
-    unsigned long long t_mark = gtid == 0 ? bt::global_ns() : 0;
-    auto lap = [&](int k) {
-        if (gtid == 0) {
-            const unsigned long long t = bt::global_ns();
-            s->ph_ns[k] += t - t_mark;
-            t_mark = t;
-        }
-    };
-    if (!barrier(a, sm)) return;
+    // the same in every CTA
+    uint32_t r = 2, r3 = 2;       // sub-round index (1 marks the zero-support edges), modulo 3
+    uint32_t epoch = 0;           // barrier arrivals so far
+    uint32_t k3 = 0;              // level number modulo 3 (slot of cand)
+    unsigned long long L = 0;     // current level
+    uint32_t nsel = 0;            // near bucket: near0, length near_ctr[nsel]
+    uint32_t *near0 = a.near_a, *near1 = a.near_b, *far0 = a.far_a, *far1 = a.far_b;
+    uint32_t near_dead = 0;       // its entries processed since it was last compacted
+    unsigned long long hi = 0;    // bound of the near bucket
+    unsigned long long live = sm.now.far_len, live_at_compress = a.m;
+    // of CTA 0's clerk
+    const unsigned long long t_start = bt::global_ns(), c_start = clock64();
+    unsigned long long t_mark = c_start, ph0 = 0, ph1 = 0;  // SM cycles
+    unsigned long long subrounds = 0, levels = 0, rebuilds = 0, compressions = 0;
 
-    uint32_t nsel = 0;         // near bucket: list near_a, length near_ctr[nsel]
     for (;;) {
         // ------------------------------------------------ level transition
-        if (s->len[r % 3] == 0) {
-            // T1: min over the near bucket (min_sup was reset in the last sub-round)
-            list_min<N32>(a, a.near_a, s->near_ctr[nsel], &s->min_sup);
-            if (!barrier(a, sm)) return;
-            if (s->min_sup == ~0ull) {
-                // T2: near is dry -> split the far bucket
-                list_min<N32>(a, a.far_a, s->far_len, &s->far_min);
-                if (!barrier(a, sm)) return;
-                const unsigned long long lo = s->far_min;
-                if (lo == ~0ull) break;  // nothing left
-                const unsigned long long hi = lo + s->delta;
-                for (uint32_t i = gtid; i < s->far_len; i += gsz) {
-                    const uint32_t e = a.far_a[i];
-                    if (a.enter[e] != 0) continue;
-                    if (sup_of<N32>(a, e) < hi) a.near_b[atomicAdd(&s->near_ctr[nsel ^ 1], 1u)] = e;
-                    else a.far_b[atomicAdd(&s->far2_len, 1u)] = e;
+        if (sm.now.len[r3] == 0) {
+            bool squeeze = false, dry = false;
+            for (;;) {
+                L = sm.now.cand[k3];
+                if (L >= hi) {
+                    // near is dry: split the far bucket
+                    const uint32_t far_len = sm.now.far_len;
+                    list_min<N32>(a, far0, far_len, &s->ctl.far_min);
+                    if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
+                    L = sm.now.far_min;
+                    if (L == ~0ull) {  // nothing left
+                        dry = true;
+                        break;
+                    }
+                    // all of it at once when a scan of it takes one entry per thread
+                    hi = live <= gsz ? ~0ull : L + sm.now.delta;
+                    for (uint32_t i = gtid; i < far_len; i += gsz) {
+                        const uint32_t e = __ldcg(far0 + i);
+                        if (__ldcg(a.enter + e) != 0) continue;
+                        if (sup_of<N32>(a, e) < hi) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
+                        else far1[atomicAdd(&s->ctl.far2_len, 1u)] = e;
+                    }
+                    if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
+                    {   // every CTA swaps its copies of the bucket pointers
+                        uint32_t *t = near0; near0 = near1; near1 = t;
+                        t = far0; far0 = far1; far1 = t;
+                    }
+                    nsel ^= 1;
+                    near_dead = 0;
+                    if (clerk) {
+                        // read again after the next barrier at the earliest
+                        s->ctl.near_ctr[nsel ^ 1] = 0;
+                        s->ctl.far_len = sm.now.far2_len;
+                        s->ctl.far2_len = 0;
+                        s->ctl.far_min = ~0ull;
+                        rebuilds++;
+                        const uint32_t near_len = sm.now.near_ctr[nsel];
+                        if (near_len > 4 * gsz && sm.now.delta > 1) s->ctl.delta = sm.now.delta >> 1;
+                        else if (near_len < gsz / 4) s->ctl.delta = sm.now.delta << 1;
+                    }
                 }
-                if (!barrier(a, sm)) return;
-                {   // every CTA swaps its copies of the bucket pointers
-                    uint32_t *t = a.near_a; a.near_a = a.near_b; a.near_b = t;
-                    t = a.far_a; a.far_a = a.far_b; a.far_b = t;
+                // frontier of sub-round r = near edges with support == L, and
+                // the lowest support above it; entries processed meanwhile are
+                // dropped from the list once they are half of it
+                k3 = next3(k3);
+                if (clerk) s->ctl.cand[next3(k3)] = ~0ull;
+                const uint32_t near_len = sm.now.near_ctr[nsel];
+                const bool compact = near_len > gsz && near_dead > near_len / 2;
+                uint32_t *front = (r & 1 ? a.list1 : a.list0);
+                SupWord<N32> low = (SupWord<N32>)~0ull;
+                for (uint32_t i = gtid; i < near_len; i += gsz) {
+                    const uint32_t e = __ldcg(near0 + i);
+                    const uint32_t en = __ldcg(a.enter + e);
+                    const SupWord<N32> v = sup_of<N32>(a, e);
+                    if (en != 0) continue;
+                    if (v == L) {
+                        list_append(a, front, &s->ctl.len[r3], s->head[r & 1], e, 0, 0, 1, r, (uint32_t)L);
+                    } else {
+                        if (v < low) low = v;
+                        if (compact) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
+                    }
                 }
-                nsel ^= 1;
-                if (gtid == 0) {
-                    s->near_ctr[nsel ^ 1] = 0;
-                    s->far_len = s->far2_len;
-                    s->far2_len = 0;
-                    s->hi = hi;
-                    s->min_sup = lo;
-                    s->far_min = ~0ull;
-                    s->rebuilds++;
-                    if (s->near_ctr[nsel] > 4 * kNearTarget && s->delta > 1) s->delta >>= 1;
-                    else if (s->near_ctr[nsel] < kNearTarget / 4) s->delta <<= 1;
+                fold_low<N32>(sm, low);
+                squeeze = (double)live <= (double)a.cfrac * (double)live_at_compress &&
+                          (double)live_at_compress >= (double)a.cfloor * (double)a.m;
+                if (!barrier(a, sm, epoch, k3, r3, r & 1, true)) return;
+                if (compact) {
+                    uint32_t *t = near0; near0 = near1; near1 = t;
+                    nsel ^= 1;
+                    near_dead = 0;
+                    if (clerk) s->ctl.near_ctr[nsel ^ 1] = 0;
                 }
-                if (!barrier(a, sm)) return;
+                // no edge at L: the minimum was of an edge that has since left;
+                // what this scan collected is exact
+                if (sm.now.len[r3] != 0) break;
             }
-            // T3: frontier of sub-round r = near edges with support == L; the
-            // rest of the live near edges are compacted into the other list
-            L = s->min_sup;
-            const uint32_t near_len = s->near_ctr[nsel];
-            uint32_t *front = a.list[r % 3];
-            for (uint32_t i = gtid; i < near_len; i += gsz) {
-                const uint32_t e = a.near_a[i];
-                if (a.enter[e] != 0) continue;
-                if (sup_of<N32>(a, e) == L) {
-                    a.enter[e] = r;
-                    a.result[e] = (uint32_t)L;
-                    front[atomicAdd(&s->len[r % 3], 1u)] = e;
-                } else {
-                    a.near_b[atomicAdd(&s->near_ctr[nsel ^ 1], 1u)] = e;
-                }
-            }
-            // T4: compression (the reference's trigger, bitruss_msp.cu:537, see cfrac)
-            const bool squeeze = (double)s->edge_num <= (double)a.cfrac * (double)s->live_at_compress &&
-                                 (double)s->live_at_compress >= (double)a.cfloor * (double)a.m;
-            if (!barrier(a, sm)) return;
-            {
-                uint32_t *t = a.near_a; a.near_a = a.near_b; a.near_b = t;
-            }
-            nsel ^= 1;
-            if (gtid == 0) {
+            if (dry) break;
+            if (clerk) {
                 s->last_level = L;
-                s->levels_seen++;
+                levels++;
                 if (L > 0xffffffffull) s->overflow = 1;
-                if (squeeze) {
-                    s->live_at_compress = (unsigned long long)s->edge_num;
-                    s->compressions++;
-                }
             }
             if (squeeze) {
+                live_at_compress = live;
+                if (clerk) compressions++;
                 compress_rows(a, r);
-                if (!barrier(a, sm)) return;
-                compute_two_hop(a);
-                epoch++;
-                if (!barrier(a, sm)) return;
+                if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
+                prepare_rows(a);
+                if (!barrier(a, sm, epoch, k3, r3, r & 1, true)) return;
             }
-            lap(0);
+            if (clerk) {
+                const unsigned long long t = clock64();
+                ph0 += t - t_mark;
+                t_mark = t;
+            }
         }
         // ------------------------------------------------ sub-round r
-        const unsigned long long sr_t0 = (a.trace && gtid == 0) ? bt::global_ns() : 0;
-        const uint32_t curr_len = s->len[r % 3];
-        const uint32_t *curr = a.list[r % 3];
-        Round rd;
+        const uint32_t curr_len = sm.now.len[r3];
+        Round<N32> rd;
         rd.r = r;
-        rd.L = L;
-        rd.hi = s->hi;
-        rd.next = a.list[(r + 1) % 3];
-        rd.next_len = &s->len[(r + 1) % 3];
-        rd.near_list = a.near_a;
-        rd.near_len = &s->near_ctr[nsel];
-        uint32_t ntasks;
-        if (curr_len <= a.local_plan) {
-            plan(a, sm, curr, curr_len, sm.lp_piv, sm.lp_anc, sm.lp_grain, sm.lp_total, sm.lp_start,
-                 blockIdx.x == 0);
-            ntasks = sm.lp_start[curr_len];
-            if (gtid == 0) s->tasks += ntasks;
-        } else {
-            if (blockIdx.x == 0) {
-                plan(a, sm, curr, curr_len, a.pl_piv, a.pl_anc, a.pl_grain, a.pl_total, a.task_start, true);
-                if (threadIdx.x == 0) {
-                    s->task_total = a.task_start[curr_len];
-                    s->tasks += s->task_total;
-                }
-            }
-            if (!barrier(a, sm)) return;
-            ntasks = s->task_total;
-        }
-        if (gtid == 0) {
+        rd.L = (SupWord<N32>)L;
+        // a bound above every support works like any other
+        rd.hi = N32 && hi > 0xffffffffull ? (SupWord<N32>)0xffffffffull : (SupWord<N32>)hi;
+        rd.next = (r & 1 ? a.list0 : a.list1);
+        rd.next_len = &s->ctl.len[next3(r3)];
+        rd.next_head = s->head[(r + 1) & 1];
+        rd.near_list = near0;
+        rd.near_len = &s->ctl.near_ctr[nsel];
+        if (clerk) {
             // slots used two sub-rounds from now; every CTA is past their last use
-            s->len[(r + 2) % 3] = 0;
-            s->task_ctr[(r + 2) % 3] = 0;
-            s->near_ctr[nsel ^ 1] = 0;  // the compaction target of the next transition
-            s->min_sup = ~0ull;
-            s->edge_num -= curr_len;
-            s->subrounds++;
+            s->ctl.len[next3(next3(r3))] = 0;
+            s->task_ctr[next3(next3(r3))] = 0;
+            subrounds++;
         }
-        if (curr_len <= a.local_plan)
-            peel_tasks<N32>(a, sm, curr, curr_len, sm.lp_piv, sm.lp_anc, sm.lp_grain, sm.lp_total, sm.lp_start,
-                       ntasks, &s->task_ctr[r % 3], rd, epoch, wk);
-        else
-            peel_tasks<N32>(a, sm, curr, curr_len, a.pl_piv, a.pl_anc, a.pl_grain, a.pl_total, a.task_start,
-                       ntasks, &s->task_ctr[r % 3], rd, epoch, wk);
-        if (!barrier(a, sm)) return;
-        if (a.trace && gtid == 0 && r < a.trace_cap) {
-            a.trace[r].t_ns = bt::global_ns() - sr_t0;
-            a.trace[r].frontier = curr_len;
-            a.trace[r].tasks = ntasks;
+        live -= curr_len;
+        near_dead += curr_len;
+        const unsigned long long task_t0 = a.trace ? bt::global_ns() : 0;
+        const unsigned long long tasks0 = sm.tasks;
+        const uint32_t probes0 = wk.probes;
+        SupWord<N32> low = (SupWord<N32>)~0ull;
+        peel<N32>(a, sm, (r & 1 ? a.list1 : a.list0), curr_len, &s->task_ctr[r3], rd, wk, low);
+        prof_mark(sm, bt::PF_PROBE);
+        fold_low<N32>(sm, low);
+        if (a.trace && r < a.trace_cap) {
+            const unsigned long long walked = warp_sum(wk.probes - probes0);
+            if ((threadIdx.x & 31) == 0) {
+                atomicMax(&a.trace[r].max_task_ns, bt::global_ns() - task_t0);
+                atomicAdd(&a.trace[r].walked, walked);
+            }
+            if (threadIdx.x == 0) atomicAdd(&a.trace[r].tasks, (uint32_t)(sm.tasks - tasks0));
         }
-        lap(1);
+        if (!barrier(a, sm, epoch, k3, next3(r3), (r + 1) & 1, true)) return;
+        if (clerk) {
+            const unsigned long long t = clock64();
+            if (a.trace && r < a.trace_cap) {
+                a.trace[r].t_ns = bt::global_ns() - task_t0;
+                a.trace[r].frontier = curr_len;
+            }
+            ph1 += t - t_mark;
+            t_mark = t;
+        }
         r++;
+        r3 = next3(r3);
     }
-    if (gtid == 0) s->done = 1;
     // flush the counters
+    if (clerk) {
+        const double ns = (double)(bt::global_ns() - t_start) / (double)(clock64() - c_start);
+        s->ph_ns[0] = (unsigned long long)((double)ph0 * ns);
+        s->ph_ns[1] = (unsigned long long)((double)ph1 * ns);
+        s->subrounds = subrounds;
+        s->levels_seen = levels;
+        s->rebuilds = rebuilds;
+        s->compressions = compressions;
+        s->done = 1;
+    }
     if (threadIdx.x == 0) {
-        for (int q = 0; q < 8; q++) atomicAdd(&s->prof[q], sm.walk.prof[q]);
-        wk.probes += sm.walk.walked;
+        for (int q = 0; q < 8; q++) atomicAdd(&s->prof[q], sm.prof[q]);
+        atomicAdd(&s->tasks, sm.tasks);
+        atomicAdd(&s->w_anchor, sm.anchor);
     }
-    for (int o = 16; o; o >>= 1) {
-        wk.mids += __shfl_xor_sync(0xffffffffu, wk.mids, o);
-        wk.probes += __shfl_xor_sync(0xffffffffu, wk.probes, o);
-        wk.hits += __shfl_xor_sync(0xffffffffu, wk.hits, o);
-        wk.decs += __shfl_xor_sync(0xffffffffu, wk.decs, o);
-    }
+    const unsigned long long probes = warp_sum(wk.probes), hits = warp_sum(wk.hits), decs = warp_sum(wk.decs);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s->w_mids, wk.mids);
-        atomicAdd(&s->w_probes, wk.probes);
-        atomicAdd(&s->w_hits, wk.hits);
-        atomicAdd(&s->w_decs, wk.decs);
+        atomicAdd(&s->w_probes, probes);
+        atomicAdd(&s->w_hits, hits);
+        atomicAdd(&s->w_decs, decs);
     }
 }
 
@@ -707,24 +880,43 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(MspArgs a) {
 // set-up kernels
 // ---------------------------------------------------------------------------
 
-__global__ void k_msp_init(uint64_t m, const unsigned long long *sup_in, unsigned long long *sup,
-                           uint32_t *sup32, uint32_t *enter, uint32_t *result, uint32_t *far_list, MspState *s) {
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
-         e += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long v = sup_in[e];
-        if (sup32) sup32[e] = (uint32_t)v;  // every support fits (checked on the host)
-        else sup[e] = v;
-        result[e] = 0;
-        if (v == 0) {
-            enter[e] = 1;  // processed first (count_es_zero, bitruss_msp.cu:38-50)
-        } else {
-            enter[e] = 0;
-            far_list[atomicAdd(&s->far_len, 1u)] = (uint32_t)e;
+constexpr int kInitThreads = 256;
+
+// Edge states, and the vertex records (the tables' places in the pool are
+// given out block by block).
+__global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsigned long long *sup_in,
+                                                           const uint32_t *off, const uint32_t *deg) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t e0 = blockIdx.x * (uint64_t)kInitThreads; e0 < a.m; e0 += (uint64_t)gridDim.x * kInitThreads) {
+        const uint64_t e = e0 + threadIdx.x;
+        const unsigned long long v = e < a.m ? sup_in[e] : 0;
+        if (e < a.m) {
+            if (a.sup32) a.sup32[e] = (uint32_t)v;  // every support fits (checked on the host)
+            else a.sup[e] = v;
+            a.result[e] = 0;
+            a.enter[e] = v == 0 ? 1 : 0;  // support 0: processed first (count_es_zero, bitruss_msp.cu:38-50)
         }
+        const uint32_t live = __ballot_sync(0xffffffffu, v != 0);
+        uint32_t at = 0;
+        if (lane == 0 && live) at = atomicAdd(&a.s->ctl.far_len, (uint32_t)__popc(live));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (v != 0) a.far_a[at + __popc(live & ((1u << lane) - 1))] = (uint32_t)e;
+    }
+    __shared__ uint32_t base;
+    __shared__ typename cub::BlockScan<uint32_t, kInitThreads>::TempStorage scan;
+    for (uint64_t x0 = blockIdx.x * (uint64_t)kInitThreads; x0 < a.n; x0 += (uint64_t)gridDim.x * kInitThreads) {
+        const uint64_t x = x0 + threadIdx.x;
+        const uint32_t d = x < a.n ? deg[x] : 0;
+        uint32_t excl, tot;
+        cub::BlockScan<uint32_t, kInitThreads>(scan).ExclusiveSum(d ? bt_row_buckets(d) : 0, excl, tot);
+        if (threadIdx.x == 0) base = atomicAdd(&a.s->pool_used, tot);
+        __syncthreads();
+        if (x < a.n) a.vrec[x] = VRec{off[x], d, base + excl, 0};
+        __syncthreads();
     }
 }
 
-__global__ void k_two_hop(MspArgs a) { compute_two_hop(a); }
+__global__ void k_msp_rows(MspArgs a) { prepare_rows(a); }
 
 }  // namespace
 
@@ -806,31 +998,24 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         if (rc != BT_OK) { release(); return rc; }        \
     } while (0)
     A(s, sizeof(MspState));
-    A(a.deg, 4 * nn);
+    A(a.vrec, sizeof(VRec) * nn);
     A(a.nbr, 8 * mm);
     A(a.eid, 8 * mm);
-    A(a.two_hop, 4 * nn);
+    A(a.pool, 32 * (g.tab_buckets ? g.tab_buckets : 1));
     // 32-bit working supports when they all fit: half the footprint and
     // 4-byte atomics for the decrements
     // (BT_MSP_WIDE=1 keeps 64-bit supports: the path graphs with a support
     // above 2^32 take, testable on small graphs)
     const char *wide = getenv("BT_MSP_WIDE");
-    if (ctx->last_sup_max <= 0xffffffffull && !(wide && *wide == '1')) A(a.sup32, 4 * mm);
+    if (ctx->last_sup_max < 0xffffffffull && !(wide && *wide == '1')) A(a.sup32, 4 * mm);
     else A(a.sup, 8 * mm);
     A(a.enter, 4 * mm);
-    A(a.list[0], 4 * mm);
-    A(a.list[1], 4 * mm);
-    A(a.list[2], 4 * mm);
+    A(a.list0, 4 * mm);
+    A(a.list1, 4 * mm);
     A(a.near_a, 4 * mm);
     A(a.near_b, 4 * mm);
     A(a.far_a, 4 * mm);
     A(a.far_b, 4 * mm);
-    A(a.pl_piv, 4 * mm);
-    A(a.pl_anc, 4 * mm);
-    A(a.pl_grain, 4 * mm);
-    A(a.pl_total, 4 * mm);
-    A(a.rowpre, 8 * mm);
-    A(a.task_start, 4 * (mm + 1));
     const char *trace_path = getenv("BT_MSP_TRACE");
     if (trace_path && *trace_path) {
         a.trace_cap = 4u << 20;
@@ -844,26 +1029,23 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         if (_e != cudaSuccess) { release(); return bt_cuda_fail(_e, #x, __FILE__, __LINE__); } \
     } while (0)
     {
+        // copied before the call returns: pageable memory
         MspState init{};
-        init.delta = 1;
-        init.hi = 0;
-        init.min_sup = ~0ull;
-        init.far_min = ~0ull;
-        init.live_at_compress = m;
+        init.ctl.delta = 1;
+        init.ctl.far_min = ~0ull;
+        for (auto &c : init.ctl.cand) c = ~0ull;
         C(cudaMemcpyAsync(s, &init, sizeof(MspState), cudaMemcpyHostToDevice, st));
-        C(cudaStreamSynchronize(st));  // `init` lives on the host stack
     }
     if (a.trace) C(cudaMemsetAsync(a.trace, 0, sizeof(TraceRow) * a.trace_cap, st));
-    C(cudaMemcpyAsync(a.deg, g.deg0, 4 * n, cudaMemcpyDeviceToDevice, st));
     C(cudaMemcpyAsync(a.nbr, g.nbr0, 8 * m, cudaMemcpyDeviceToDevice, st));
     C(cudaMemcpyAsync(a.eid, g.eid0, 8 * m, cudaMemcpyDeviceToDevice, st));
     a.s = s;
     a.n = g.n;
     a.m = m;
     a.exact = exact ? 1u : 0u;
-    a.min_grain = ctx->msp_schedule[0] ? ctx->msp_schedule[0] : kMspMinGrain;
-    a.tasks_per_cta = ctx->msp_schedule[1] ? ctx->msp_schedule[1] : kMspTasksPerCta;
-    a.local_plan = ctx->msp_schedule[2] ? std::min(ctx->msp_schedule[2], kLocalPlan) : kLocalPlan;
+    a.inv_task = 1.0f / (float)(ctx->msp_schedule[0] ? ctx->msp_schedule[0] : kMspMinGrain);
+    a.chunks_per_cta = ctx->msp_schedule[1] ? ctx->msp_schedule[1] : kMspTasksPerCta;
+    a.local_plan = std::min(ctx->msp_schedule[2] ? ctx->msp_schedule[2] : kMspLocalPlan, kEdges);
     a.wait_ns = wait_limit_ns();
     // Row compaction: whenever the live edges have halved since the last
     // compaction.  The reference also stops compacting once fewer than a tenth
@@ -881,27 +1063,14 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
             a.cfloor = fl;
         }
     }
-    a.off = g.off;
     a.ends = g.ends;
-    a.hub_base = g.hub_base;
-    a.hub_mask = g.hub_mask;
-    a.hub_pool = g.hub_pool;
-    const unsigned blk = 256, cap = (unsigned)ctx->sm_count * 8;
+    const unsigned blk = kInitThreads, cap = (unsigned)ctx->sm_count * 8;
     if (m) {
-        k_msp_init<<<(unsigned)std::min<uint64_t>((m + blk - 1) / blk, cap), blk, 0, st>>>(
-            m, (const unsigned long long *)ctx->sup, a.sup, a.sup32, a.enter, a.result, a.far_a, s); bt_note_launches(1);
-        C(cudaGetLastError());
-    }
-    // edge_num = live edges
-    MspState h0;
-    {
-        C(cudaMemcpyAsync(&h0, s, sizeof(MspState), cudaMemcpyDeviceToHost, st));
-        C(cudaStreamSynchronize(st));
-        h0.edge_num = h0.far_len;
-        C(cudaMemcpyAsync(s, &h0, sizeof(MspState), cudaMemcpyHostToDevice, st));
-    }
-    if (n) {
-        k_two_hop<<<(unsigned)std::min<uint64_t>((n * 32 + blk - 1) / blk, cap), blk, 0, st>>>(a); bt_note_launches(1);
+        const uint64_t most = std::max<uint64_t>(m, n);
+        k_msp_init<<<(unsigned)std::min<uint64_t>((most + blk - 1) / blk, cap), blk, 0, st>>>(
+            a, (const unsigned long long *)ctx->sup, g.off, g.deg0);
+        k_msp_rows<<<(unsigned)std::min<uint64_t>((n * 32 + blk - 1) / blk, cap), blk, 0, st>>>(a);
+        bt_note_launches(2);
         C(cudaGetLastError());
     }
     // cooperative persistent launch
@@ -974,7 +1143,7 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     ctx->stats[3] = h.tasks;
     ctx->stats[5] = h.levels_seen;
     ctx->stats[6] = h.rebuilds;
-    ctx->work[0] = h.w_mids;
+    ctx->work[0] = h.tasks;
     ctx->work[1] = h.w_probes;
     ctx->work[2] = h.w_anchor;
     ctx->work[3] = h.w_hits;

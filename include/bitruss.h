@@ -156,17 +156,17 @@ double bt_ctx_phase_ms(const bt_ctx *ctx, const char *phase);
  * (4 when every support fits 32 bits, else 8); [18] edge recomputations of
  * the last hidx over all its rounds, [19] 1 if it started from the exact
  * peel's values, 0 if from the supports; [20..27] SM cycles per CTA of the peeling
- * kernel by step: task lookup, anchor staging, slice load, probe pass, hit
- * pass, flushes, grid-barrier waits, other work.  After a batched call, [1] is
+ * kernel by step, where the kernel has it: [23] tasks, [26] grid-barrier waits
+ * and plans, [27] the rest.  After a batched call, [1] is
  * the sub-rounds summed over its arenas and [7] the number of arenas. */
 bt_status bt_ctx_stats(const bt_ctx *ctx, uint64_t *out, int n);
 
 /* ---- peeling schedule and its autotuner ------------------------------- */
 
-/* The msp task schedule.  min_grain: probe positions per peel task, at least;
- * tasks_per_cta: a sub-round's work is cut into about this many tasks per
- * CTA; local_plan: frontiers of at most this many edges (<= 512) are planned
- * by every CTA without a grid barrier.  0 keeps the built-in value (2048, 2,
+/* The msp task schedule.  min_grain: probe positions a peel task (one warp)
+ * should hold; tasks_per_cta: chunks per CTA that a frontier too large to be
+ * planned whole is cut into; local_plan: frontiers of at most this many edges
+ * (<= 512) are planned whole by every CTA.  0 keeps the built-in value (64, 2,
  * 512).  Results never depend on the schedule.  No reference counterpart (the
  * reference launches one block per frontier edge: bitruss_msp.cu:286-291). */
 bt_status bt_ctx_set_msp_schedule(bt_ctx *ctx, uint32_t min_grain, uint32_t tasks_per_cta,

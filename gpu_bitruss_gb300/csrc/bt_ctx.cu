@@ -7,6 +7,7 @@
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_segmented_sort.cuh>
 
+#include <algorithm>
 #include <cstring>
 #include <atomic>
 #include <mutex>
@@ -335,13 +336,13 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
     g.n = n;
     g.m = m;
     g.u_num = hg->u_num;
-    uint32_t maxd = 0;
     for (uint32_t x = 0; x < n; x++) {
         const uint32_t d = hg->degrees[x];
-        maxd = d > maxd ? d : maxd;
+        uint32_t &side = x < g.u_num ? g.max_deg_u : g.max_deg_l;
+        side = d > side ? d : side;
         if (d) g.tab_buckets += bt_row_buckets(d);
     }
-    g.max_deg = maxd;
+    g.max_deg = std::max(g.max_deg_u, g.max_deg_l);
 
     // persistent arrays
     BT_TRY(ctx_alloc_t(ctx, &g.off, (uint64_t)n + 1));

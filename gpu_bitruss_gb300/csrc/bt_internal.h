@@ -77,6 +77,7 @@ struct DevGraph {
     uint32_t n = 0, u_num = 0;
     uint64_t m = 0;
     uint32_t max_deg = 0;
+    uint32_t max_deg_u = 0, max_deg_l = 0;  // largest degree of either side
     uint32_t *off = nullptr;    // n+1 row starts
     uint32_t *deg0 = nullptr;   // n   degree
     uint32_t *nbr0 = nullptr;   // 2m  neighbour rank, ascending per row
@@ -128,6 +129,7 @@ struct bt_ctx {
     // scratch reused across calls
     void *scratch = nullptr;
     uint64_t scratch_bytes = 0;
+    uint64_t zero_counters = 0;  // leading counters of the scratch known to be zero (bt_count.cu)
 
     double phase_ms[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
     uint64_t stats[8] = {0};
@@ -158,6 +160,9 @@ bt_status ctx_alloc_t(bt_ctx *ctx, T **p, uint64_t count) {
 }
 bt_status ctx_scratch(bt_ctx *ctx, uint64_t bytes, void **p);
 void ctx_release_graph(bt_ctx *ctx);
+
+// most bytes the counting kernel's scratch takes (bt_count.cu)
+uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide);
 
 // algorithm entry points implemented in the .cu files
 bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *g);

@@ -654,19 +654,24 @@ __device__ __forceinline__ void compress_rows(const MspArgs &a, uint32_t r) {
     }
 }
 
-// Position total and table of every row; one warp per vertex.
-__device__ __forceinline__ void prepare_rows(const MspArgs &a) {
+// Position total (from the degrees `deg` gives) and table of row x, by one warp.
+template <class Deg>
+__device__ __forceinline__ void prepare_row(const MspArgs &a, uint32_t x, uint32_t off, uint32_t d, uint32_t tab,
+                                            Deg deg) {
     const uint32_t lane = threadIdx.x & 31;
+    unsigned long long hop = 0;
+    for (uint32_t j = lane; j < d; j += 32) hop += deg(a.nbr[off + j]);
+    hop = warp_sum(hop);
+    if (lane == 0) a.vrec[x].hop = hop > 0xffffffffull ? 0xffffffffu : (uint32_t)hop;
+    bt::row_build(a.pool, tab, d, a.nbr + off, a.eid + off);
+}
+
+__device__ __forceinline__ void prepare_rows(const MspArgs &a) {
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t x = warp; x < a.n; x += nw) {
         const VRec v = load_vrec(a.vrec + x);
-        if (v.deg == 0) continue;
-        unsigned long long hop = 0;
-        for (uint32_t j = lane; j < v.deg; j += 32) hop += __ldcg(&a.vrec[a.nbr[v.off + j]].deg);
-        hop = warp_sum(hop);
-        if (lane == 0) a.vrec[x].hop = hop > 0xffffffffull ? 0xffffffffu : (uint32_t)hop;
-        bt::row_build(a.pool, v.tab, v.deg, a.nbr + v.off, a.eid + v.off);
+        if (v.deg) prepare_row(a, x, v.off, v.deg, v.tab, [&](uint32_t y) { return __ldcg(&a.vrec[y].deg); });
     }
 }
 
@@ -882,8 +887,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
 
 constexpr int kInitThreads = 256;
 
-// Edge states, and the vertex records (the tables' places in the pool are
-// given out block by block).
+// Edge states, vertex records and row tables (the tables' places in the pool
+// are given out block by block).
 __global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsigned long long *sup_in,
                                                            const uint32_t *off, const uint32_t *deg) {
     const uint32_t lane = threadIdx.x & 31;
@@ -902,21 +907,28 @@ __global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsi
         at = __shfl_sync(0xffffffffu, at, 0);
         if (v != 0) a.far_a[at + __popc(live & ((1u << lane) - 1))] = (uint32_t)e;
     }
+    // vertices: a block's tables are laid out first, then its warps build them
     __shared__ uint32_t base;
+    __shared__ uint32_t s_tab[kInitThreads];
     __shared__ typename cub::BlockScan<uint32_t, kInitThreads>::TempStorage scan;
-    for (uint64_t x0 = blockIdx.x * (uint64_t)kInitThreads; x0 < a.n; x0 += (uint64_t)gridDim.x * kInitThreads) {
-        const uint64_t x = x0 + threadIdx.x;
+    const uint64_t step = gridDim.x;  // a block's vertices lie this far apart: ranks follow degree
+    for (uint64_t x0 = blockIdx.x; x0 < a.n; x0 += step * kInitThreads) {
+        const uint64_t x = x0 + step * threadIdx.x;
         const uint32_t d = x < a.n ? deg[x] : 0;
         uint32_t excl, tot;
         cub::BlockScan<uint32_t, kInitThreads>(scan).ExclusiveSum(d ? bt_row_buckets(d) : 0, excl, tot);
         if (threadIdx.x == 0) base = atomicAdd(&a.s->pool_used, tot);
         __syncthreads();
+        s_tab[threadIdx.x] = base + excl;
         if (x < a.n) a.vrec[x] = VRec{off[x], d, base + excl, 0};
+        __syncthreads();
+        for (uint32_t k = threadIdx.x >> 5; k < kInitThreads && x0 + step * k < a.n; k += kInitThreads / 32) {
+            const uint32_t y = (uint32_t)(x0 + step * k), dy = deg[y];
+            if (dy) prepare_row(a, y, off[y], dy, s_tab[k], [&](uint32_t z) { return __ldg(deg + z); });
+        }
         __syncthreads();
     }
 }
-
-__global__ void k_msp_rows(MspArgs a) { prepare_rows(a); }
 
 }  // namespace
 
@@ -1066,11 +1078,11 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     a.ends = g.ends;
     const unsigned blk = kInitThreads, cap = (unsigned)ctx->sm_count * 8;
     if (m) {
-        const uint64_t most = std::max<uint64_t>(m, n);
-        k_msp_init<<<(unsigned)std::min<uint64_t>((most + blk - 1) / blk, cap), blk, 0, st>>>(
+        // a thread per edge, a warp per row
+        const uint64_t blocks = std::max<uint64_t>((m + blk - 1) / blk, (n * 32 + blk - 1) / blk);
+        k_msp_init<<<(unsigned)std::min<uint64_t>(blocks, cap), blk, 0, st>>>(
             a, (const unsigned long long *)ctx->sup, g.off, g.deg0);
-        k_msp_rows<<<(unsigned)std::min<uint64_t>((n * 32 + blk - 1) / blk, cap), blk, 0, st>>>(a);
-        bt_note_launches(2);
+        bt_note_launches(1);
         C(cudaGetLastError());
     }
     // cooperative persistent launch

@@ -95,7 +95,7 @@ uint64_t bt_job_footprint(uint64_t n, uint64_t m, uint64_t hub_slots, uint64_t t
                           uint64_t count_ctas, bool peel) {
     const uint64_t resident = 36 * m + 24 * n + 8 * hub_slots + (1u << 16);
     const uint64_t upload = 32 * m + 52 * n + (16 * m + 24 * n + (4u << 20));
-    const uint64_t count = 8 * span * count_ctas + (1u << 20);
+    const uint64_t count = bt_count_bytes(m, span, count_ctas, true) + (1u << 16);
     const uint64_t msp = peel ? 52 * m + 16 * n + 32 * tab_buckets + (1u << 16) : 0;
     return resident + std::max(upload, count + msp);
 }

@@ -82,6 +82,10 @@
 namespace {
 
 using bt::kEmpty;
+using bt::load_vrec;
+using bt::VRec;
+using bt::warp_inclusive;
+using bt::warp_sum;
 constexpr int kThreads = 512;
 constexpr uint32_t kWarps = kThreads / 32;
 constexpr uint32_t kEdges = kMspLocalPlan;  // frontier edges a CTA plans at once
@@ -111,7 +115,7 @@ struct MspState {
     uint32_t pool_used;            // row table buckets given out
     uint32_t done, overflow;
     unsigned long long ph_ns[2];   // CTA 0's time in: level transitions, sub-rounds
-    unsigned long long prof[8];    // SM cycles summed over CTAs, by step (bt::PF_*)
+    unsigned long long prof[8];    // SM cycles summed over CTAs, by step (PF_*)
     // statistics
     unsigned long long subrounds, compressions, tasks, levels_seen, rebuilds;
     // work counters (algorithmic bytes): tasks, row positions walked, anchor
@@ -130,12 +134,6 @@ struct TraceRow {
     unsigned long long max_task_ns; // longest CTA
     unsigned long long walked;      // row positions walked
     uint32_t frontier, tasks;
-};
-
-// Per vertex, one 16-byte load: row start, live degree, first bucket of its
-// row table, and the row's position total (sum of its neighbours' degrees).
-struct __align__(16) VRec {
-    uint32_t off, deg, tab, hop;
 };
 
 struct MspArgs {
@@ -177,16 +175,6 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
         v = t < v ? t : v;
     }
     return v;
-}
-
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ VRec load_vrec(const VRec *p) {
-    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(p));
-    return VRec{q.x, q.y, q.z, q.w};
 }
 
 // The peel rule for one butterfly seen from frontier edge uv; returns a 3-bit
@@ -310,10 +298,13 @@ struct Smem {
     uint32_t chunk, total, next_task;
     Control now;                           // the control words as of the last barrier
     unsigned long long tasks, anchor;      // counters of this CTA
-    unsigned long long prof_t, prof[8];    // see bt::PF_*
+    unsigned long long prof_t, prof[8];    // see PF_*
 };
 
 constexpr uint32_t kPivIsV = 0x80000000u;  // the pivot is the edge's V end
+
+// Steps of the time accounting (indices of the published counters).
+enum { PF_PROBE = 3, PF_BARRIER = 6, PF_OTHER = 7 };
 
 // Time accounting and bookkeeping are done by a CTA's last thread: the first
 // warp plans and has the first task, so it is on the longest path.
@@ -342,16 +333,6 @@ __device__ __forceinline__ uint4 load_control(const MspArgs &a, Smem &sm, uint32
 // ---------------------------------------------------------------------------
 // peel
 // ---------------------------------------------------------------------------
-
-__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
-    const uint32_t lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= (uint32_t)o) v += t;
-    }
-    return v;
-}
 
 // Plan frontier edge e as entry i: orientation and tasks; returns their number.
 //  * The pivot is the endpoint whose row's position total is smaller; both
@@ -434,7 +415,7 @@ __device__ __forceinline__ void plan_block(const MspArgs &a, Smem &sm, const uin
 __device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm, uint32_t &epoch, uint32_t k3, uint32_t r3,
                                         uint32_t list, bool plan) {
     __syncthreads();
-    prof_mark(sm, bt::PF_OTHER);
+    prof_mark(sm, PF_OTHER);
     int ok = 1;
     if (threadIdx.x < 32) {
         const unsigned long long low = sm.low;
@@ -454,7 +435,7 @@ __device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm, uint32_t &ep
             plan_warp(a, sm, len, head, a.nblocks * kWarps, blockIdx.x == 0);
     }
     ok = __syncthreads_and(ok);
-    prof_mark(sm, bt::PF_BARRIER);
+    prof_mark(sm, PF_BARRIER);
     return ok != 0;
 }
 
@@ -663,7 +644,7 @@ __device__ __forceinline__ void prepare_row(const MspArgs &a, uint32_t x, uint32
     for (uint32_t j = lane; j < d; j += 32) hop += deg(a.nbr[off + j]);
     hop = warp_sum(hop);
     if (lane == 0) a.vrec[x].hop = hop > 0xffffffffull ? 0xffffffffu : (uint32_t)hop;
-    bt::row_build(a.pool, tab, d, a.nbr + off, a.eid + off);
+    bt::row_build(a.pool, tab, d, a.nbr + off, [&](uint32_t j) { return a.eid[off + j]; });
 }
 
 __device__ __forceinline__ void prepare_rows(const MspArgs &a) {
@@ -834,7 +815,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
         const uint32_t probes0 = wk.probes;
         SupWord<N32> low = (SupWord<N32>)~0ull;
         peel<N32>(a, sm, (r & 1 ? a.list1 : a.list0), curr_len, &s->task_ctr[r3], rd, wk, low);
-        prof_mark(sm, bt::PF_PROBE);
+        prof_mark(sm, PF_PROBE);
         fold_low<N32>(sm, low);
         if (a.trace && r < a.trace_cap) {
             const unsigned long long walked = warp_sum(wk.probes - probes0);

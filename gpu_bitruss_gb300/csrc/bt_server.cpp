@@ -56,7 +56,7 @@ struct Request {
     const bt_graph *g = nullptr;
     int op = 0;
     void *out = nullptr;
-    uint64_t hub_slots = 0, tab_buckets = 0;
+    uint64_t tab_buckets = 0;
     Clock::time_point t_submit, t_admit, t_done;
     bool admitted = false, done = false;
     bt_status status = BT_OK;
@@ -75,25 +75,14 @@ uint64_t tab_buckets_of(const bt_graph *g) {
     return s;
 }
 
-uint64_t hub_slots_of(const bt_graph *g) {
-    uint64_t s = 0;
-    for (uint32_t d : g->degrees)
-        if (d > 256) {  // bt::kHubMinDeg
-            uint64_t sz = 64;
-            while (sz < 2ull * d) sz <<= 1;
-            s += sz;
-        }
-    return s;
-}
-
 }  // namespace
 
 // Device bytes a job on an arena of these sizes allocates at its peak (every
 // array of dev_build_graph, dev_ebfc and dev_msp; CUB temporaries bounded
 // above).  count_ctas: resident CTAs of the counting kernel.
-uint64_t bt_job_footprint(uint64_t n, uint64_t m, uint64_t hub_slots, uint64_t tab_buckets, uint64_t span,
+uint64_t bt_job_footprint(uint64_t n, uint64_t m, uint64_t tab_buckets, uint64_t span,
                           uint64_t count_ctas, bool peel) {
-    const uint64_t resident = 36 * m + 24 * n + 8 * hub_slots + (1u << 16);
+    const uint64_t resident = 36 * m + 16 * n + (1u << 16);
     const uint64_t upload = 32 * m + 52 * n + (16 * m + 24 * n + (4u << 20));
     const uint64_t count = bt_count_bytes(m, span, count_ctas, true) + (1u << 16);
     const uint64_t msp = peel ? 52 * m + 16 * n + 32 * tab_buckets + (1u << 16) : 0;
@@ -106,16 +95,15 @@ extern "C" bt_status bt_job_bytes(bt_ctx *ctx, const bt_graph *const *graphs, ui
                                   uint64_t *bytes) {
     if (!ctx || !bytes || (count && !graphs)) return bt_fail(BT_ERR_INVALID, "null argument");
     if (op < BT_OP_BFC || op > BT_OP_MSP_EXACT) return bt_fail(BT_ERR_INVALID, "unknown op");
-    uint64_t n = 0, m = 0, hub = 0, tab = 0, span = 0;
+    uint64_t n = 0, m = 0, tab = 0, span = 0;
     for (uint32_t i = 0; i < count; i++) {
         if (!graphs[i]) return bt_fail(BT_ERR_INVALID, "null graph");
         n += graphs[i]->n;
         m += graphs[i]->m;
-        hub += hub_slots_of(graphs[i]);
         tab += tab_buckets_of(graphs[i]);
         span = std::max<uint64_t>(span, graphs[i]->n);
     }
-    *bytes = bt_job_footprint(n, m, hub, tab, span, (uint64_t)dev_count_ctas(ctx), kind_of(op) != 0);
+    *bytes = bt_job_footprint(n, m, tab, span, (uint64_t)dev_count_ctas(ctx), kind_of(op) != 0);
     return BT_OK;
 }
 
@@ -136,15 +124,14 @@ struct bt_server {
     uint64_t completed = 0, batches = 0, batched_requests = 0;
 
     uint64_t footprint(const std::vector<ReqPtr> &job) const {
-        uint64_t n = 0, m = 0, hub = 0, tab = 0, span = 0;
+        uint64_t n = 0, m = 0, tab = 0, span = 0;
         for (const auto &r : job) {
             n += r->g->n;
             m += r->g->m;
-            hub += r->hub_slots;
             tab += r->tab_buckets;
             span = std::max<uint64_t>(span, r->g->n);
         }
-        return bt_job_footprint(n, m, hub, tab, span, count_ctas, kind_of(job[0]->op) != 0);
+        return bt_job_footprint(n, m, tab, span, count_ctas, kind_of(job[0]->op) != 0);
     }
 
     // pick a job (lock held); empty if nothing can start now
@@ -372,7 +359,6 @@ extern "C" bt_status bt_server_submit(bt_server *s, const bt_graph *g, int op, v
     r->g = g;
     r->op = op;
     r->out = out;
-    r->hub_slots = hub_slots_of(g);
     r->tab_buckets = tab_buckets_of(g);
     {
         std::lock_guard<std::mutex> lk(s->mu);

@@ -11,14 +11,13 @@
 // each graph's priority ranks contiguous (the counting kernel then sizes its
 // per-CTA counters by the largest graph instead of the whole arena).
 //
-// Why the results are per-graph exact: a butterfly never spans two graphs, so
-// a frontier edge of graph i only decrements edges of graph i, and the msp
-// rule compares edge ids of one butterfly only (their order survives the
-// offset).  Each level's frontier of the union is the union of the graphs'
-// frontiers; a graph whose own frontier is empty at a sub-round takes no part
-// in it.  So every edge receives the value it receives when its graph is
-// peeled alone, and a graph's level count (the last level with a frontier
-// edge) is the largest bitruss number among its edges.
+// Why the results are per-graph exact: every graph is peeled by itself, by a team
+// of CTAs, on its own ranks and edges of the arena.  (Peeling the union in one
+// go would give the same: a butterfly never spans two graphs, so a frontier
+// edge of graph i only decrements edges of graph i, and the msp rule compares
+// edge ids of one butterfly only, whose order survives the offset.)  A graph's
+// level count (the last level with a frontier edge) is the largest bitruss
+// number among its edges.
 #include <omp.h>
 
 #include <algorithm>
@@ -65,6 +64,8 @@ bt_status pack_range(const bt_graph *const *graphs, uint32_t first, uint32_t las
     out->seg_max_n = max_n;
     try {
         out->segment.assign(out->n, 0);
+        out->seg_n.resize(k);
+        out->seg_m.resize(k);
         out->offsets.assign((size_t)out->n + 1, 0);
         out->degrees.assign(out->n, 0);
         out->neighbors.resize(2 * M);
@@ -72,6 +73,10 @@ bt_status pack_range(const bt_graph *const *graphs, uint32_t first, uint32_t las
         out->edges.resize(2 * M);
     } catch (const std::bad_alloc &) {
         return bt_fail(BT_ERR_HOST_MEMORY, "host allocation of the arena failed");
+    }
+    for (uint32_t i = 0; i < k; i++) {
+        out->seg_n[i] = graphs[first + i]->n;
+        out->seg_m[i] = (uint32_t)graphs[first + i]->m;
     }
     out->edge_support_raw.clear();
     out->bitruss_raw.clear();

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <string>
 
 #include "bt_device.cuh"
@@ -325,6 +326,22 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
         if (d) g.tab_buckets += bt_row_buckets(d);
     }
     g.max_deg = std::max(g.max_deg_u, g.max_deg_l);
+    try {
+        g.spans.reserve(hg->segment.empty() ? 1 : hg->seg_n.size());
+    } catch (const std::bad_alloc &) {
+        return bt_fail(BT_ERR_HOST_MEMORY, "host allocation failed");
+    }
+    if (hg->segment.empty()) {
+        g.spans.push_back({0, n, 0, (uint32_t)m});
+    } else {
+        uint32_t v0 = 0, e0 = 0;
+        for (size_t i = 0; i < hg->seg_n.size(); i++) {
+            g.spans.push_back({v0, hg->seg_n[i], e0, hg->seg_m[i]});
+            v0 += hg->seg_n[i];
+            e0 += hg->seg_m[i];
+        }
+        if (v0 != n || e0 != m) return bt_fail(BT_ERR_INVALID, "arena spans do not match the arena");
+    }
 
     // persistent arrays
     BT_TRY(ctx_alloc_t(ctx, &g.off, (uint64_t)n + 1));

@@ -62,6 +62,7 @@ struct bt_graph {
     // and the vertex count of the largest graph
     std::vector<uint32_t> segment;
     uint32_t seg_max_n = 0;
+    std::vector<uint32_t> seg_n, seg_m;  // vertices and edges of every graph
 };
 
 // ---------------------------------------------------------------------------
@@ -88,6 +89,11 @@ struct DevGraph {
     // batched arena: ranks are grouped by graph; seg_base[r] = first rank of
     // r's graph (NULL for one graph); cnt_span = vertices of the largest graph
     uint32_t *seg_base = nullptr;
+    // every graph's ranks [v0, v0 + n) and edges [e0, e0 + m) (one entry for one graph)
+    struct Span {
+        uint32_t v0, n, e0, m;
+    };
+    std::vector<Span> spans;
     uint32_t cnt_span = 0;
 };
 

@@ -21,7 +21,9 @@
 //
 // GB300 design: one cooperative persistent kernel runs the whole level /
 // sub-round loop on the device (the reference pays 3 host syncs and ~9m bytes
-// of copies per sub-round, :527-533).
+// of copies per sub-round, :527-533).  One graph has the whole grid; the graphs
+// of a batched arena are peeled side by side, each by a team of CTAs with its
+// own barrier, lists and levels ("grid" below is the team's).
 //
 // What bounds it: the chain.  A decomposition is tens of thousands of
 // sub-rounds that depend on one another, most of them of 10^3 to 10^5 row
@@ -70,11 +72,17 @@
 // longer and only hub rows of 500k edges and more gained (3%).
 // Grid barriers are bounded by a time limit; an expired wait sets an error and
 // the kernel returns.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <condition_variable>
+#include <functional>
 #include <mutex>
+#include <new>
+#include <queue>
 #include <type_traits>
+#include <vector>
 
 #include "bt_device.cuh"
 #include "bt_internal.h"
@@ -104,23 +112,50 @@ struct Control {
 constexpr uint32_t kControlWords = sizeof(Control) / 4;
 static_assert(kControlWords <= 32, "the control words are loaded by one warp");
 
+// The state of one graph's peel (zero but for far_len when the kernel starts; the
+// team that takes it sets the rest).
 struct MspState {
-    bt::Barrier bar;
     __align__(128) Control ctl;
     // the first entries of the two frontier lists as (edge, U end, V end, 0):
     // what a short frontier's plan needs, written by whoever appends
     uint4 head[2][32];
     uint32_t task_ctr[3];          // chunk counters by sub-round index mod 3
-    unsigned long long last_level; // last level with a non-empty frontier
+};
+
+// A graph of the arena: its ranks [v0, v1) and edges [e0, e0 + m).
+struct Job {
+    uint32_t v0, v1, e0, m;
+};
+
+// CTAs [cta0, cta0 + size) that peel one graph after another.
+struct __align__(128) TeamState {
+    bt::Barrier bar;
+    uint32_t job, cta0, size;
+};
+
+// Of the whole launch.
+struct MspShared {
+    uint32_t queue;                // jobs given out past the teams' first ones
     uint32_t pool_used;            // row table buckets given out
-    uint32_t done, overflow;
-    unsigned long long ph_ns[2];   // CTA 0's time in: level transitions, sub-rounds
+    uint32_t done, overflow, error;
+    unsigned long long last_level; // the largest last level with a non-empty frontier
+    unsigned long long ph_ns[2];   // the first team's time in: level transitions, sub-rounds
     unsigned long long prof[8];    // SM cycles summed over CTAs, by step (PF_*)
     // statistics
     unsigned long long subrounds, compressions, tasks, levels_seen, rebuilds;
-    // work counters (algorithmic bytes): tasks, row positions walked, anchor
-    // slots of the peeled edges, butterflies found, decrements
-    unsigned long long w_tasks, w_probes, w_anchor, w_hits, w_decs;
+    // work counters (algorithmic bytes): row positions walked, anchor slots of
+    // the peeled edges, butterflies found, decrements
+    unsigned long long w_probes, w_anchor, w_hits, w_decs;
+};
+
+// A CTA's place in its team, and the graph the team is on.
+struct Team {
+    uint32_t rank, size;
+    bt::Barrier *bar;
+    MspState *s;
+    Job job;
+    __device__ __forceinline__ uint32_t thread() const { return rank * kThreads + threadIdx.x; }
+    __device__ __forceinline__ uint32_t threads() const { return size * kThreads; }
 };
 
 // Counters of one thread.
@@ -137,8 +172,13 @@ struct TraceRow {
 };
 
 struct MspArgs {
-    MspState *s;
-    uint32_t n, nblocks, exact;
+    MspShared *sh;
+    TeamState *teams;
+    MspState *states;               // per job
+    const Job *jobs;                // largest first
+    uint32_t njobs, nteams;
+    const uint32_t *team_of;        // per CTA
+    uint32_t n, exact;
     uint32_t chunks_per_cta, local_plan;  // schedule, with inv_task (results do not depend on it)
     // row compaction trigger: compact when the live edges fall to cfrac of
     // the live edges at the last compaction, while those were at least
@@ -322,11 +362,11 @@ __device__ __forceinline__ void prof_mark(Smem &sm, int k) {
 // first warp (the caller synchronises the block).
 // One request per CTA: the same word read by all 2,432 warps of the grid at
 // once is served one request at a time by its L2 slice (about a microsecond).
-__device__ __forceinline__ uint4 load_control(const MspArgs &a, Smem &sm, uint32_t list) {
-    const uint4 head = __ldcg(&a.s->head[list][threadIdx.x]);
+__device__ __forceinline__ uint4 load_control(const MspState *s, Smem &sm, uint32_t list) {
+    const uint4 head = __ldcg(&s->head[list][threadIdx.x]);
     if (threadIdx.x < kControlWords)
         reinterpret_cast<uint32_t *>(&sm.now)[threadIdx.x] =
-            __ldcg(reinterpret_cast<const uint32_t *>(&a.s->ctl) + threadIdx.x);
+            __ldcg(reinterpret_cast<const uint32_t *>(&s->ctl) + threadIdx.x);
     return head;
 }
 
@@ -409,10 +449,10 @@ __device__ __forceinline__ void plan_block(const MspArgs &a, Smem &sm, const uin
     __syncthreads();
 }
 
-// Grid barrier.  Publishes the CTA's running minimum to cand[k3], refreshes
+// Barrier of the team.  Publishes the CTA's running minimum to cand[k3], refreshes
 // sm.now, and with `plan` plans the next frontier (length len[r3], list `list`)
 // when it is a short one: its entries come with the control words.
-__device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm, uint32_t &epoch, uint32_t k3, uint32_t r3,
+__device__ __forceinline__ bool barrier(const MspArgs &a, const Team &t, Smem &sm, uint32_t &epoch, uint32_t k3, uint32_t r3,
                                         uint32_t list, bool plan) {
     __syncthreads();
     prof_mark(sm, PF_OTHER);
@@ -422,17 +462,18 @@ __device__ __forceinline__ bool barrier(const MspArgs &a, Smem &sm, uint32_t &ep
         __syncwarp();
         if (threadIdx.x == 0) {
             // (sm.now is of the last barrier: cand only falls meanwhile)
-            if (low < sm.now.cand[k3]) atomicMin(&a.s->ctl.cand[k3], low);
+            if (low < sm.now.cand[k3]) atomicMin(&t.s->ctl.cand[k3], low);
             sm.low = ~0ull;
         }
         __syncwarp();
-        epoch += a.nblocks;
-        ok = bt::barrier_wait(&a.s->bar, epoch, a.wait_ns);
-        const uint4 head = load_control(a, sm, list);
+        epoch += t.size;
+        ok = bt::barrier_wait(t.bar, epoch, a.wait_ns);
+        if (!ok) a.sh->error = bt::ERR_TIMEOUT;
+        const uint4 head = load_control(t.s, sm, list);
         __syncwarp();
         const uint32_t len = sm.now.len[r3];
         if (plan && len - 1 < 32 && len <= a.local_plan)
-            plan_warp(a, sm, len, head, a.nblocks * kWarps, blockIdx.x == 0);
+            plan_warp(a, sm, len, head, t.size * kWarps, t.rank == 0);
     }
     ok = __syncthreads_and(ok);
     prof_mark(sm, PF_BARRIER);
@@ -558,9 +599,9 @@ __device__ __forceinline__ void run_tasks(const MspArgs &a, Smem &sm, uint32_t c
 // Peel the frontier curr[0, len): one sub-round without its barrier (which
 // has planned it already when it is short).
 template <bool N32>
-__device__ __forceinline__ void peel(const MspArgs &a, Smem &sm, const uint32_t *curr, uint32_t len, uint32_t *ctr,
+__device__ __forceinline__ void peel(const MspArgs &a, const Team &t, Smem &sm, const uint32_t *curr, uint32_t len, uint32_t *ctr,
                                      const Round<N32> &rd, Work &wk, SupWord<N32> &low) {
-    const uint32_t rank = blockIdx.x, size = a.nblocks;
+    const uint32_t rank = t.rank, size = t.size;
     // a frontier that every CTA plans whole, its tasks dealt to all CTAs, or
     // chunks of it that a CTA plans and runs alone: its first is its own
     // rank, the rest come from the counter
@@ -588,11 +629,11 @@ __device__ __forceinline__ void peel(const MspArgs &a, Smem &sm, const uint32_t 
 // level transition helpers
 // ---------------------------------------------------------------------------
 
-// Minimum support over the live entries of `list` (grid-wide atomicMin).
+// Minimum support over the live entries of `list` (team-wide atomicMin).
 template <bool N32>
-__device__ __forceinline__ void list_min(const MspArgs &a, const uint32_t *list, uint32_t len, unsigned long long *out) {
+__device__ __forceinline__ void list_min(const MspArgs &a, const Team &t, const uint32_t *list, uint32_t len, unsigned long long *out) {
     unsigned long long v = ~0ull;
-    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+    const uint32_t gtid = t.thread(), gsz = t.threads();
     for (uint32_t i = gtid; i < len; i += gsz) {
         const uint32_t e = __ldcg(list + i);
         const uint32_t en = __ldcg(a.enter + e);
@@ -605,11 +646,10 @@ __device__ __forceinline__ void list_min(const MspArgs &a, const uint32_t *list,
 
 // Drop processed edges (enter in (0, r)) from every row; one warp per vertex,
 // in place.
-__device__ __forceinline__ void compress_rows(const MspArgs &a, uint32_t r) {
+__device__ __forceinline__ void compress_rows(const MspArgs &a, const Team &t, uint32_t r) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t x = warp; x < a.n; x += nw) {
+    const uint32_t nw = t.threads() >> 5;
+    for (uint32_t x = t.job.v0 + (t.thread() >> 5); x < t.job.v1; x += nw) {
         const uint32_t b = a.vrec[x].off, d = a.vrec[x].deg;
         uint32_t w = 0;
         for (uint32_t j0 = 0; j0 < d; j0 += 32) {
@@ -647,10 +687,9 @@ __device__ __forceinline__ void prepare_row(const MspArgs &a, uint32_t x, uint32
     bt::row_build(a.pool, tab, d, a.nbr + off, [&](uint32_t j) { return a.eid[off + j]; });
 }
 
-__device__ __forceinline__ void prepare_rows(const MspArgs &a) {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t x = warp; x < a.n; x += nw) {
+__device__ __forceinline__ void prepare_rows(const MspArgs &a, const Team &t) {
+    const uint32_t nw = t.threads() >> 5;
+    for (uint32_t x = t.job.v0 + (t.thread() >> 5); x < t.job.v1; x += nw) {
         const VRec v = load_vrec(a.vrec + x);
         if (v.deg) prepare_row(a, x, v.off, v.deg, v.tab, [&](uint32_t y) { return __ldcg(&a.vrec[y].deg); });
     }
@@ -664,201 +703,235 @@ template <bool N32>
 __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ MspArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
-    MspState *s = a.s;
     if (threadIdx.x == 0) {
         sm.low = ~0ull;
         sm.tasks = sm.anchor = 0;
         for (int k = 0; k < 8; k++) sm.prof[k] = 0;
     }
     if (is_clerk()) sm.prof_t = clock64();
-    if (threadIdx.x < 32) load_control(a, sm, 0);
     sm.dec[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
-    const bool clerk = blockIdx.x == 0 && is_clerk();
+    Team t;
+    const uint32_t team_index = a.team_of[blockIdx.x];
+    TeamState *team = a.teams + team_index;
+    t.size = team->size;
+    t.rank = blockIdx.x - team->cta0;
+    t.bar = &team->bar;
+    const uint32_t gtid = t.thread(), gsz = t.threads();
+    const bool clerk = t.rank == 0 && is_clerk();
     Work wk;
-    // the same in every CTA
-    uint32_t r = 2, r3 = 2;       // sub-round index (1 marks the zero-support edges), modulo 3
-    uint32_t epoch = 0;           // barrier arrivals so far
-    uint32_t k3 = 0;              // level number modulo 3 (slot of cand)
-    unsigned long long L = 0;     // current level
-    uint32_t nsel = 0;            // near bucket: near0, length near_ctr[nsel]
-    uint32_t *near0 = a.near_a, *near1 = a.near_b, *far0 = a.far_a, *far1 = a.far_b;
-    uint32_t near_dead = 0;       // its entries processed since it was last compacted
-    unsigned long long hi = 0;    // bound of the near bucket
-    unsigned long long live = sm.now.far_len, live_at_compress = a.m;
-    // of CTA 0's clerk
+    uint32_t epoch = 0;               // barrier arrivals so far (the same in every CTA of the team)
+    // of the team's clerk
     const unsigned long long t_start = bt::global_ns(), c_start = clock64();
     unsigned long long t_mark = c_start, ph0 = 0, ph1 = 0;  // SM cycles
     unsigned long long subrounds = 0, levels = 0, rebuilds = 0, compressions = 0;
 
-    for (;;) {
-        // ------------------------------------------------ level transition
-        if (sm.now.len[r3] == 0) {
-            bool squeeze = false, dry = false;
-            for (;;) {
-                L = sm.now.cand[k3];
-                if (L >= hi) {
-                    // near is dry: split the far bucket
-                    const uint32_t far_len = sm.now.far_len;
-                    list_min<N32>(a, far0, far_len, &s->ctl.far_min);
-                    if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
-                    L = sm.now.far_min;
-                    if (L == ~0ull) {  // nothing left
-                        dry = true;
-                        break;
+    for (bool first = true;; first = false) {
+        // ---------------------------------------------------- the next graph
+        if (t.rank == 0 && threadIdx.x == 0) {
+            const uint32_t q = first ? team_index : a.nteams + atomicAdd(&a.sh->queue, 1u);
+            if (q < a.njobs) {
+                Control &c = a.states[q].ctl;
+                c.delta = 1;
+                c.far_min = c.cand[0] = c.cand[1] = c.cand[2] = ~0ull;
+            }
+            team->job = q;
+        }
+        __syncthreads();
+        int ok = 1;
+        if (threadIdx.x < 32) {
+            epoch += t.size;
+            ok = bt::barrier_wait(t.bar, epoch, a.wait_ns);
+            if (!ok) a.sh->error = bt::ERR_TIMEOUT;
+            const uint32_t q = __ldcg(&team->job);
+            if (threadIdx.x == 0) sm.chunk = q;
+            if (q < a.njobs) load_control(a.states + q, sm, 0);
+        }
+        if (!__syncthreads_and(ok)) return;
+        const uint32_t q = sm.chunk;
+        if (q >= a.njobs) break;
+        MspState *s = t.s = a.states + q;
+        t.job = a.jobs[q];
+        // the same in every CTA of the team
+        uint32_t r = 2, r3 = 2;       // sub-round index (1 marks the zero-support edges), modulo 3
+        uint32_t k3 = 0;              // level number modulo 3 (slot of cand)
+        unsigned long long L = 0;     // current level
+        uint32_t nsel = 0;            // near bucket: near0, length near_ctr[nsel]
+        const uint32_t e0 = t.job.e0; // the lists of a graph lie at its edges' place
+        uint32_t *near0 = a.near_a + e0, *near1 = a.near_b + e0, *far0 = a.far_a + e0, *far1 = a.far_b + e0;
+        uint32_t near_dead = 0;       // its entries processed since it was last compacted
+        unsigned long long hi = 0;    // bound of the near bucket
+        unsigned long long live = sm.now.far_len, live_at_compress = t.job.m;
+        for (;;) {
+            // ------------------------------------------------ level transition
+            if (sm.now.len[r3] == 0) {
+                bool squeeze = false, dry = false;
+                for (;;) {
+                    L = sm.now.cand[k3];
+                    if (L >= hi) {
+                        // near is dry: split the far bucket
+                        const uint32_t far_len = sm.now.far_len;
+                        list_min<N32>(a, t, far0, far_len, &s->ctl.far_min);
+                        if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                        L = sm.now.far_min;
+                        if (L == ~0ull) {  // nothing left
+                            dry = true;
+                            break;
+                        }
+                        // all of it at once when a scan of it takes one entry per thread
+                        hi = live <= gsz ? ~0ull : L + sm.now.delta;
+                        for (uint32_t i = gtid; i < far_len; i += gsz) {
+                            const uint32_t e = __ldcg(far0 + i);
+                            if (__ldcg(a.enter + e) != 0) continue;
+                            if (sup_of<N32>(a, e) < hi) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
+                            else far1[atomicAdd(&s->ctl.far2_len, 1u)] = e;
+                        }
+                        if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                        {   // every CTA swaps its copies of the bucket pointers
+                            uint32_t *t = near0; near0 = near1; near1 = t;
+                            t = far0; far0 = far1; far1 = t;
+                        }
+                        nsel ^= 1;
+                        near_dead = 0;
+                        if (clerk) {
+                            // read again after the next barrier at the earliest
+                            s->ctl.near_ctr[nsel ^ 1] = 0;
+                            s->ctl.far_len = sm.now.far2_len;
+                            s->ctl.far2_len = 0;
+                            s->ctl.far_min = ~0ull;
+                            rebuilds++;
+                            const uint32_t near_len = sm.now.near_ctr[nsel];
+                            if (near_len > 4 * gsz && sm.now.delta > 1) s->ctl.delta = sm.now.delta >> 1;
+                            else if (near_len < gsz / 4) s->ctl.delta = sm.now.delta << 1;
+                        }
                     }
-                    // all of it at once when a scan of it takes one entry per thread
-                    hi = live <= gsz ? ~0ull : L + sm.now.delta;
-                    for (uint32_t i = gtid; i < far_len; i += gsz) {
-                        const uint32_t e = __ldcg(far0 + i);
-                        if (__ldcg(a.enter + e) != 0) continue;
-                        if (sup_of<N32>(a, e) < hi) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
-                        else far1[atomicAdd(&s->ctl.far2_len, 1u)] = e;
+                    // frontier of sub-round r = near edges with support == L, and
+                    // the lowest support above it; entries processed meanwhile are
+                    // dropped from the list once they are half of it
+                    k3 = next3(k3);
+                    if (clerk) s->ctl.cand[next3(k3)] = ~0ull;
+                    const uint32_t near_len = sm.now.near_ctr[nsel];
+                    const bool compact = near_len > gsz && near_dead > near_len / 2;
+                    uint32_t *front = ((r & 1 ? a.list1 : a.list0) + e0);
+                    SupWord<N32> low = (SupWord<N32>)~0ull;
+                    for (uint32_t i = gtid; i < near_len; i += gsz) {
+                        const uint32_t e = __ldcg(near0 + i);
+                        const uint32_t en = __ldcg(a.enter + e);
+                        const SupWord<N32> v = sup_of<N32>(a, e);
+                        if (en != 0) continue;
+                        if (v == L) {
+                            list_append(a, front, &s->ctl.len[r3], s->head[r & 1], e, 0, 0, 1, r, (uint32_t)L);
+                        } else {
+                            if (v < low) low = v;
+                            if (compact) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
+                        }
                     }
-                    if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
-                    {   // every CTA swaps its copies of the bucket pointers
+                    fold_low<N32>(sm, low);
+                    squeeze = (double)live <= (double)a.cfrac * (double)live_at_compress &&
+                              (double)live_at_compress >= (double)a.cfloor * (double)t.job.m;
+                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, true)) return;
+                    if (compact) {
                         uint32_t *t = near0; near0 = near1; near1 = t;
-                        t = far0; far0 = far1; far1 = t;
+                        nsel ^= 1;
+                        near_dead = 0;
+                        if (clerk) s->ctl.near_ctr[nsel ^ 1] = 0;
                     }
-                    nsel ^= 1;
-                    near_dead = 0;
-                    if (clerk) {
-                        // read again after the next barrier at the earliest
-                        s->ctl.near_ctr[nsel ^ 1] = 0;
-                        s->ctl.far_len = sm.now.far2_len;
-                        s->ctl.far2_len = 0;
-                        s->ctl.far_min = ~0ull;
-                        rebuilds++;
-                        const uint32_t near_len = sm.now.near_ctr[nsel];
-                        if (near_len > 4 * gsz && sm.now.delta > 1) s->ctl.delta = sm.now.delta >> 1;
-                        else if (near_len < gsz / 4) s->ctl.delta = sm.now.delta << 1;
-                    }
+                    // no edge at L: the minimum was of an edge that has since left;
+                    // what this scan collected is exact
+                    if (sm.now.len[r3] != 0) break;
                 }
-                // frontier of sub-round r = near edges with support == L, and
-                // the lowest support above it; entries processed meanwhile are
-                // dropped from the list once they are half of it
-                k3 = next3(k3);
-                if (clerk) s->ctl.cand[next3(k3)] = ~0ull;
-                const uint32_t near_len = sm.now.near_ctr[nsel];
-                const bool compact = near_len > gsz && near_dead > near_len / 2;
-                uint32_t *front = (r & 1 ? a.list1 : a.list0);
-                SupWord<N32> low = (SupWord<N32>)~0ull;
-                for (uint32_t i = gtid; i < near_len; i += gsz) {
-                    const uint32_t e = __ldcg(near0 + i);
-                    const uint32_t en = __ldcg(a.enter + e);
-                    const SupWord<N32> v = sup_of<N32>(a, e);
-                    if (en != 0) continue;
-                    if (v == L) {
-                        list_append(a, front, &s->ctl.len[r3], s->head[r & 1], e, 0, 0, 1, r, (uint32_t)L);
-                    } else {
-                        if (v < low) low = v;
-                        if (compact) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
-                    }
+                if (dry) break;
+                if (clerk) {
+                    atomicMax(&a.sh->last_level, L);
+                    levels++;
+                    if (L > 0xffffffffull) a.sh->overflow = 1;
                 }
-                fold_low<N32>(sm, low);
-                squeeze = (double)live <= (double)a.cfrac * (double)live_at_compress &&
-                          (double)live_at_compress >= (double)a.cfloor * (double)a.m;
-                if (!barrier(a, sm, epoch, k3, r3, r & 1, true)) return;
-                if (compact) {
-                    uint32_t *t = near0; near0 = near1; near1 = t;
-                    nsel ^= 1;
-                    near_dead = 0;
-                    if (clerk) s->ctl.near_ctr[nsel ^ 1] = 0;
+                if (squeeze) {
+                    live_at_compress = live;
+                    if (clerk) compressions++;
+                    compress_rows(a, t, r);
+                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                    prepare_rows(a, t);
+                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, true)) return;
                 }
-                // no edge at L: the minimum was of an edge that has since left;
-                // what this scan collected is exact
-                if (sm.now.len[r3] != 0) break;
+                if (clerk) {
+                    const unsigned long long t = clock64();
+                    ph0 += t - t_mark;
+                    t_mark = t;
+                }
             }
-            if (dry) break;
+            // ------------------------------------------------ sub-round r
+            const uint32_t curr_len = sm.now.len[r3];
+            Round<N32> rd;
+            rd.r = r;
+            rd.L = (SupWord<N32>)L;
+            // a bound above every support works like any other
+            rd.hi = N32 && hi > 0xffffffffull ? (SupWord<N32>)0xffffffffull : (SupWord<N32>)hi;
+            rd.next = ((r & 1 ? a.list0 : a.list1) + e0);
+            rd.next_len = &s->ctl.len[next3(r3)];
+            rd.next_head = s->head[(r + 1) & 1];
+            rd.near_list = near0;
+            rd.near_len = &s->ctl.near_ctr[nsel];
             if (clerk) {
-                s->last_level = L;
-                levels++;
-                if (L > 0xffffffffull) s->overflow = 1;
+                // slots used two sub-rounds from now; every CTA is past their last use
+                s->ctl.len[next3(next3(r3))] = 0;
+                s->task_ctr[next3(next3(r3))] = 0;
+                subrounds++;
             }
-            if (squeeze) {
-                live_at_compress = live;
-                if (clerk) compressions++;
-                compress_rows(a, r);
-                if (!barrier(a, sm, epoch, k3, r3, r & 1, false)) return;
-                prepare_rows(a);
-                if (!barrier(a, sm, epoch, k3, r3, r & 1, true)) return;
+            live -= curr_len;
+            near_dead += curr_len;
+            const unsigned long long task_t0 = a.trace ? bt::global_ns() : 0;
+            const unsigned long long tasks0 = sm.tasks;
+            const uint32_t probes0 = wk.probes;
+            SupWord<N32> low = (SupWord<N32>)~0ull;
+            peel<N32>(a, t, sm, ((r & 1 ? a.list1 : a.list0) + e0), curr_len, &s->task_ctr[r3], rd, wk, low);
+            prof_mark(sm, PF_PROBE);
+            fold_low<N32>(sm, low);
+            if (a.trace && r < a.trace_cap) {
+                const unsigned long long walked = warp_sum(wk.probes - probes0);
+                if ((threadIdx.x & 31) == 0) {
+                    atomicMax(&a.trace[r].max_task_ns, bt::global_ns() - task_t0);
+                    atomicAdd(&a.trace[r].walked, walked);
+                }
+                if (threadIdx.x == 0) atomicAdd(&a.trace[r].tasks, (uint32_t)(sm.tasks - tasks0));
             }
+            if (!barrier(a, t, sm, epoch, k3, next3(r3), (r + 1) & 1, true)) return;
             if (clerk) {
                 const unsigned long long t = clock64();
-                ph0 += t - t_mark;
+                if (a.trace && r < a.trace_cap) {
+                    a.trace[r].t_ns = bt::global_ns() - task_t0;
+                    a.trace[r].frontier = curr_len;
+                }
+                ph1 += t - t_mark;
                 t_mark = t;
             }
+            r++;
+            r3 = next3(r3);
         }
-        // ------------------------------------------------ sub-round r
-        const uint32_t curr_len = sm.now.len[r3];
-        Round<N32> rd;
-        rd.r = r;
-        rd.L = (SupWord<N32>)L;
-        // a bound above every support works like any other
-        rd.hi = N32 && hi > 0xffffffffull ? (SupWord<N32>)0xffffffffull : (SupWord<N32>)hi;
-        rd.next = (r & 1 ? a.list0 : a.list1);
-        rd.next_len = &s->ctl.len[next3(r3)];
-        rd.next_head = s->head[(r + 1) & 1];
-        rd.near_list = near0;
-        rd.near_len = &s->ctl.near_ctr[nsel];
-        if (clerk) {
-            // slots used two sub-rounds from now; every CTA is past their last use
-            s->ctl.len[next3(next3(r3))] = 0;
-            s->task_ctr[next3(next3(r3))] = 0;
-            subrounds++;
-        }
-        live -= curr_len;
-        near_dead += curr_len;
-        const unsigned long long task_t0 = a.trace ? bt::global_ns() : 0;
-        const unsigned long long tasks0 = sm.tasks;
-        const uint32_t probes0 = wk.probes;
-        SupWord<N32> low = (SupWord<N32>)~0ull;
-        peel<N32>(a, sm, (r & 1 ? a.list1 : a.list0), curr_len, &s->task_ctr[r3], rd, wk, low);
-        prof_mark(sm, PF_PROBE);
-        fold_low<N32>(sm, low);
-        if (a.trace && r < a.trace_cap) {
-            const unsigned long long walked = warp_sum(wk.probes - probes0);
-            if ((threadIdx.x & 31) == 0) {
-                atomicMax(&a.trace[r].max_task_ns, bt::global_ns() - task_t0);
-                atomicAdd(&a.trace[r].walked, walked);
-            }
-            if (threadIdx.x == 0) atomicAdd(&a.trace[r].tasks, (uint32_t)(sm.tasks - tasks0));
-        }
-        if (!barrier(a, sm, epoch, k3, next3(r3), (r + 1) & 1, true)) return;
-        if (clerk) {
-            const unsigned long long t = clock64();
-            if (a.trace && r < a.trace_cap) {
-                a.trace[r].t_ns = bt::global_ns() - task_t0;
-                a.trace[r].frontier = curr_len;
-            }
-            ph1 += t - t_mark;
-            t_mark = t;
-        }
-        r++;
-        r3 = next3(r3);
+        if (clerk) atomicAdd(&a.sh->done, 1u);
     }
     // flush the counters
     if (clerk) {
-        const double ns = (double)(bt::global_ns() - t_start) / (double)(clock64() - c_start);
-        s->ph_ns[0] = (unsigned long long)((double)ph0 * ns);
-        s->ph_ns[1] = (unsigned long long)((double)ph1 * ns);
-        s->subrounds = subrounds;
-        s->levels_seen = levels;
-        s->rebuilds = rebuilds;
-        s->compressions = compressions;
-        s->done = 1;
+        if (blockIdx.x == 0) {
+            const double ns = (double)(bt::global_ns() - t_start) / (double)(clock64() - c_start);
+            a.sh->ph_ns[0] = (unsigned long long)((double)ph0 * ns);
+            a.sh->ph_ns[1] = (unsigned long long)((double)ph1 * ns);
+        }
+        atomicAdd(&a.sh->subrounds, subrounds);
+        atomicAdd(&a.sh->levels_seen, levels);
+        atomicAdd(&a.sh->rebuilds, rebuilds);
+        atomicAdd(&a.sh->compressions, compressions);
     }
     if (threadIdx.x == 0) {
-        for (int q = 0; q < 8; q++) atomicAdd(&s->prof[q], sm.prof[q]);
-        atomicAdd(&s->tasks, sm.tasks);
-        atomicAdd(&s->w_anchor, sm.anchor);
+        for (int q = 0; q < 8; q++) atomicAdd(&a.sh->prof[q], sm.prof[q]);
+        atomicAdd(&a.sh->tasks, sm.tasks);
+        atomicAdd(&a.sh->w_anchor, sm.anchor);
     }
     const unsigned long long probes = warp_sum(wk.probes), hits = warp_sum(wk.hits), decs = warp_sum(wk.decs);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s->w_probes, probes);
-        atomicAdd(&s->w_hits, hits);
-        atomicAdd(&s->w_decs, decs);
+        atomicAdd(&a.sh->w_probes, probes);
+        atomicAdd(&a.sh->w_hits, hits);
+        atomicAdd(&a.sh->w_decs, decs);
     }
 }
 
@@ -869,9 +942,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
 constexpr int kInitThreads = 256;
 
 // Edge states, vertex records and row tables (the tables' places in the pool
-// are given out block by block).
+// are given out block by block).  by_edge: (first edge, job) of every graph, by
+// first edge.
 __global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsigned long long *sup_in,
-                                                           const uint32_t *off, const uint32_t *deg) {
+                                                           const uint32_t *off, const uint32_t *deg,
+                                                           const uint2 *by_edge) {
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t e0 = blockIdx.x * (uint64_t)kInitThreads; e0 < a.m; e0 += (uint64_t)gridDim.x * kInitThreads) {
         const uint64_t e = e0 + threadIdx.x;
@@ -882,11 +957,24 @@ __global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsi
             a.result[e] = 0;
             a.enter[e] = v == 0 ? 1 : 0;  // support 0: processed first (count_es_zero, bitruss_msp.cu:38-50)
         }
-        const uint32_t live = __ballot_sync(0xffffffffu, v != 0);
+        // the far list of the edge's graph: one counter update per warp and graph
+        uint32_t q = 0;
+        if (a.njobs > 1) {
+            uint32_t hi = a.njobs;
+            while (hi - q > 1) {  // the last graph whose first edge is at or below e
+                const uint32_t md = (q + hi) >> 1;
+                if (by_edge[md].x <= e) q = md;
+                else hi = md;
+            }
+        }
+        const uint32_t peers = __match_any_sync(0xffffffffu, v != 0 ? q : kEmpty);
         uint32_t at = 0;
-        if (lane == 0 && live) at = atomicAdd(&a.s->ctl.far_len, (uint32_t)__popc(live));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (v != 0) a.far_a[at + __popc(live & ((1u << lane) - 1))] = (uint32_t)e;
+        const uint32_t leader = __ffs(peers) - 1;
+        if (v != 0 && lane == leader)
+            at = atomicAdd(&a.states[a.njobs > 1 ? by_edge[q].y : 0].ctl.far_len, (uint32_t)__popc(peers));
+        at = __shfl_sync(0xffffffffu, at, leader);
+        if (v != 0)
+            a.far_a[(a.njobs > 1 ? by_edge[q].x : 0) + at + __popc(peers & ((1u << lane) - 1))] = (uint32_t)e;
     }
     // vertices: a block's tables are laid out first, then its warps build them
     __shared__ uint32_t base;
@@ -898,7 +986,7 @@ __global__ void __launch_bounds__(kInitThreads) k_msp_init(MspArgs a, const unsi
         const uint32_t d = x < a.n ? deg[x] : 0;
         uint32_t excl, tot;
         cub::BlockScan<uint32_t, kInitThreads>(scan).ExclusiveSum(d ? bt_row_buckets(d) : 0, excl, tot);
-        if (threadIdx.x == 0) base = atomicAdd(&a.s->pool_used, tot);
+        if (threadIdx.x == 0) base = atomicAdd(&a.sh->pool_used, tot);
         __syncthreads();
         s_tab[threadIdx.x] = base + excl;
         if (x < a.n) a.vrec[x] = VRec{off[x], d, base + excl, 0};
@@ -953,6 +1041,64 @@ struct CtaSlots {
 };
 }  // namespace
 
+// Sizes of the teams.  One graph takes all CTAs.  A batch is peeled by teams
+// that take graphs one after another, largest first: a graph's peel is a chain
+// of sub-rounds that does not get shorter with more CTAs (6.5 us each), beside
+// the row positions walked, which do (150 per us and CTA).  Both grow with
+// powers of the edge count; the figures are those of Chung-Lu graphs of mean
+// degree 8 (421 / 1,876 / 8,235 sub-rounds and 0.6 / 15 / 390 million positions
+// at 10k / 100k / 1M edges; the estimate was within 10% for teams of 1 to 19),
+// and only the balance of the two matters here.  Numbers of teams, with sizes in
+// proportion to a power of their first graph's positions, are played through
+// and the one that ends first is taken.  48 graphs of 1k to 100k edges: 23 ms, with
+// the best equal sizes (8 or 9 CTAs) 26, as one chain of the union's sub-rounds 45.
+static std::vector<uint32_t> plan_teams(const std::vector<Job> &jobs, uint32_t ctas) {
+    std::vector<uint32_t> best{ctas};
+    if (jobs.size() < 2) return best;
+    std::vector<double> chain, walk;
+    for (const Job &j : jobs) {
+        chain.push_back(6.5 * 421 * pow(j.m / 1e4, 0.65));
+        walk.push_back(6.3e5 / 150 * pow(j.m / 1e4, 1.4));
+    }
+    double best_us = 0;
+    for (size_t q = 0; q < jobs.size(); q++) best_us += chain[q] + walk[q] / ctas;
+    for (uint32_t teams = 2; teams <= ctas && teams <= jobs.size(); teams += std::max(1u, teams / 3)) {
+        for (double power : {0.0, 0.5}) {
+            std::vector<uint32_t> size(teams);
+            double sum = 0;
+            for (uint32_t t = 0; t < teams; t++) sum += pow(walk[t], power);
+            uint32_t used = 0;
+            for (uint32_t t = 0; t < teams; t++) {
+                size[t] = std::max(1u, (uint32_t)(ctas * pow(walk[t], power) / sum));
+                used += size[t];
+            }
+            for (uint32_t t = 0; used < ctas; t = (t + 1) % teams, used++) size[t]++;
+            for (uint32_t t = 0; used > ctas; t = (t + 1) % teams)
+                if (size[t] > 1) size[t]--, used--;
+            std::priority_queue<std::pair<double, uint32_t>, std::vector<std::pair<double, uint32_t>>,
+                                std::greater<std::pair<double, uint32_t>>> free_at;
+            double last = 0;
+            for (size_t q = 0; q < jobs.size() && (last < best_us); q++) {
+                double at = 0;
+                uint32_t t = (uint32_t)q;
+                if (q >= teams) {
+                    at = free_at.top().first;
+                    t = free_at.top().second;
+                    free_at.pop();
+                }
+                at += chain[q] + walk[q] / size[t];
+                last = std::max(last, at);
+                free_at.push({at, t});
+            }
+            if (last < best_us) {
+                best_us = last;
+                best = size;
+            }
+        }
+    }
+    return best;
+}
+
 static unsigned long long wait_limit_ns() {
     const char *us = getenv("BT_WAIT_LIMIT_US");
     if (us && strtoull(us, nullptr, 10) > 0) return strtoull(us, nullptr, 10) * 1000ull;
@@ -962,7 +1108,7 @@ static unsigned long long wait_limit_ns() {
     return ms * 1000000ull;
 }
 
-bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
+static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     uint64_t dummy = 0;
     BT_TRY(dev_ebfc(ctx, true, &dummy));
     DevGraph &g = ctx->g;
@@ -981,8 +1127,17 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         for (void *p : owned) ctx_free(ctx, p);
         owned.clear();
     };
+    // the graphs to peel, largest first, and how many CTAs peel each
+    std::vector<Job> jobs;
+    std::vector<uint2> by_edge;
+    for (const auto &sp : g.spans)
+        if (sp.m) jobs.push_back(Job{sp.v0, sp.v0 + sp.n, sp.e0, sp.m});
+    std::stable_sort(jobs.begin(), jobs.end(), [](const Job &x, const Job &y) { return x.m > y.m; });
+    for (uint32_t q = 0; q < jobs.size(); q++) by_edge.push_back(make_uint2(jobs[q].e0, q));
+    std::sort(by_edge.begin(), by_edge.end(), [](const uint2 &x, const uint2 &y) { return x.x < y.x; });
+    const uint32_t njobs = (uint32_t)jobs.size();
     MspArgs a{};
-    MspState *s = nullptr;
+    uint2 *d_by_edge = nullptr;
     const uint64_t mm = m ? m : 1, nn = n ? n : 1;
     bt_status rc = BT_OK;
 #define A(p, bytes)                                       \
@@ -990,7 +1145,10 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         rc = alloc((void **)&(p), (bytes));               \
         if (rc != BT_OK) { release(); return rc; }        \
     } while (0)
-    A(s, sizeof(MspState));
+    A(a.sh, sizeof(MspShared));
+    A(a.states, sizeof(MspState) * (njobs ? njobs : 1));
+    A(a.jobs, sizeof(Job) * (njobs ? njobs : 1));
+    A(d_by_edge, sizeof(uint2) * (njobs ? njobs : 1));
     A(a.vrec, sizeof(VRec) * nn);
     A(a.nbr, 8 * mm);
     A(a.eid, 8 * mm);
@@ -1010,29 +1168,52 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     A(a.far_a, 4 * mm);
     A(a.far_b, 4 * mm);
     const char *trace_path = getenv("BT_MSP_TRACE");
-    if (trace_path && *trace_path) {
+    if (trace_path && *trace_path && njobs == 1) {
         a.trace_cap = 4u << 20;
         A(a.trace, sizeof(TraceRow) * a.trace_cap);
     }
-#undef A
     a.result = ctx->result;
 #define C(x)                                                                  \
     do {                                                                      \
         cudaError_t _e = (x);                                                 \
         if (_e != cudaSuccess) { release(); return bt_cuda_fail(_e, #x, __FILE__, __LINE__); } \
     } while (0)
-    {
-        // copied before the call returns: pageable memory
-        MspState init{};
-        init.ctl.delta = 1;
-        init.ctl.far_min = ~0ull;
-        for (auto &c : init.ctl.cand) c = ~0ull;
-        C(cudaMemcpyAsync(s, &init, sizeof(MspState), cudaMemcpyHostToDevice, st));
+    // cooperative persistent launch: its CTAs, in teams
+    const size_t smem = sizeof(Smem);
+    const void *kfn = a.sup32 ? (const void *)k_msp<true> : (const void *)k_msp<false>;
+    C(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    C(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kThreads, smem));
+    if (per_sm < 1) { release(); return bt_fail(BT_ERR_CUDA, "msp kernel does not fit on an SM"); }
+    const uint32_t capacity = (uint32_t)(ctx->sm_count * per_sm);
+    const uint32_t ctas = ctx->peel_ctas && ctx->peel_ctas < capacity ? ctx->peel_ctas : capacity;
+    const std::vector<uint32_t> sizes = plan_teams(jobs, ctas);
+    std::vector<TeamState> teams(sizes.size());
+    std::vector<uint32_t> team_of;
+    for (uint32_t t = 0; t < sizes.size(); t++) {
+        teams[t] = TeamState{};
+        teams[t].cta0 = (uint32_t)team_of.size();
+        teams[t].size = sizes[t];
+        team_of.insert(team_of.end(), sizes[t], t);
+    }
+    const uint32_t nblocks = (uint32_t)team_of.size();
+    a.nteams = (uint32_t)sizes.size();
+    A(a.teams, sizeof(TeamState) * teams.size());
+    A(a.team_of, 4 * team_of.size());
+#undef A
+    C(cudaMemsetAsync(a.sh, 0, sizeof(MspShared), st));
+    // (these are copied before the calls return: pageable memory)
+    C(cudaMemcpyAsync(a.teams, teams.data(), sizeof(TeamState) * teams.size(), cudaMemcpyHostToDevice, st));
+    C(cudaMemcpyAsync((void *)a.team_of, team_of.data(), 4 * team_of.size(), cudaMemcpyHostToDevice, st));
+    C(cudaMemsetAsync(a.states, 0, sizeof(MspState) * (njobs ? njobs : 1), st));
+    if (njobs) {
+        C(cudaMemcpyAsync((void *)a.jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st));
+        C(cudaMemcpyAsync(d_by_edge, by_edge.data(), sizeof(uint2) * njobs, cudaMemcpyHostToDevice, st));
     }
     if (a.trace) C(cudaMemsetAsync(a.trace, 0, sizeof(TraceRow) * a.trace_cap, st));
     C(cudaMemcpyAsync(a.nbr, g.nbr0, 8 * m, cudaMemcpyDeviceToDevice, st));
     C(cudaMemcpyAsync(a.eid, g.eid0, 8 * m, cudaMemcpyDeviceToDevice, st));
-    a.s = s;
+    a.njobs = njobs;
     a.n = g.n;
     a.m = m;
     a.exact = exact ? 1u : 0u;
@@ -1062,19 +1243,10 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         // a thread per edge, a warp per row
         const uint64_t blocks = std::max<uint64_t>((m + blk - 1) / blk, (n * 32 + blk - 1) / blk);
         k_msp_init<<<(unsigned)std::min<uint64_t>(blocks, cap), blk, 0, st>>>(
-            a, (const unsigned long long *)ctx->sup, g.off, g.deg0);
+            a, (const unsigned long long *)ctx->sup, g.off, g.deg0, d_by_edge);
         bt_note_launches(1);
         C(cudaGetLastError());
     }
-    // cooperative persistent launch
-    const size_t smem = sizeof(Smem);
-    const void *kfn = a.sup32 ? (const void *)k_msp<true> : (const void *)k_msp<false>;
-    C(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    C(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kThreads, smem));
-    if (per_sm < 1) { release(); return bt_fail(BT_ERR_CUDA, "msp kernel does not fit on an SM"); }
-    const uint32_t capacity = (uint32_t)(ctx->sm_count * per_sm);
-    a.nblocks = ctx->peel_ctas && ctx->peel_ctas < capacity ? ctx->peel_ctas : capacity;
     if (ctx->device < 0 || ctx->device >= kMaxPoolDevices) {
         release();
         return bt_fail(BT_ERR_INVALID, "device index out of range");
@@ -1083,10 +1255,10 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     CtaSlots slots;
     NvtxRange range("k_msp");
     if (m) {
-        slots.acquire(ctx->device, ctx->sm_count, (int)((a.nblocks + per_sm - 1) / per_sm));
+        slots.acquire(ctx->device, ctx->sm_count, (int)((nblocks + per_sm - 1) / per_sm));
         void *params[] = {&a};
         cudaEventRecord(ctx->ev[4], st);
-        cudaError_t le = cudaLaunchCooperativeKernel(kfn, dim3(a.nblocks), dim3(kThreads), params, smem, st);
+        cudaError_t le = cudaLaunchCooperativeKernel(kfn, dim3(nblocks), dim3(kThreads), params, smem, st);
         if (le == cudaSuccess) le = cudaGetLastError();
         if (le != cudaSuccess) {
             slots.release();
@@ -1097,9 +1269,9 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         bt_note_launches(1);
     }
     cudaEventRecord(e1, st);
-    MspState h{};
+    MspShared h{};
     {
-        cudaError_t ce = cudaMemcpyAsync(&h, s, sizeof(MspState), cudaMemcpyDeviceToHost, st);
+        cudaError_t ce = cudaMemcpyAsync(&h, a.sh, sizeof(MspShared), cudaMemcpyDeviceToHost, st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
         slots.release();
         if (ce != cudaSuccess) {
@@ -1126,10 +1298,10 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     if (m) cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]);
     ctx->phase_ms[PH_PEEL] = ms;
     release();
-    if (h.bar.error == bt::ERR_TIMEOUT)
+    if (h.error == bt::ERR_TIMEOUT)
         return bt_fail(BT_ERR_TIMEOUT, "msp: a grid barrier wait exceeded its time limit");
     if (h.overflow) return bt_fail(BT_ERR_OVERFLOW, "msp: a bitruss number exceeds uint32");
-    if (m && !h.done) return bt_fail(BT_ERR_CUDA, "msp kernel ended without finishing");
+    if (h.done != njobs) return bt_fail(BT_ERR_CUDA, "msp kernel ended without finishing");
     ctx->stats[0] = h.last_level;
     ctx->stats[1] = h.subrounds;
     ctx->stats[2] = h.compressions;
@@ -1146,8 +1318,16 @@ bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     ctx->work[7] = h.ph_ns[1];
     ctx->work[8] = 0;
     ctx->work[9] = a.sup32 ? 4 : 8;  // bytes per working support (and per decrement)
-    for (int q = 0; q < 8; q++) ctx->prof[q] = h.prof[q] / (a.nblocks ? a.nblocks : 1);
+    for (int q = 0; q < 8; q++) ctx->prof[q] = h.prof[q] / (nblocks ? nblocks : 1);
     ctx->last_result = 2;
     if (levels) *levels = (uint32_t)h.last_level;
     return BT_OK;
+}
+
+bt_status dev_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
+    try {
+        return run_msp(ctx, exact, levels);
+    } catch (const std::bad_alloc &) {
+        return bt_fail(BT_ERR_HOST_MEMORY, "host allocation failed");
+    }
 }

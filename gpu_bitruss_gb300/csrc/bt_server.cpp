@@ -81,11 +81,11 @@ uint64_t tab_buckets_of(const bt_graph *g) {
 // array of dev_build_graph, dev_ebfc and dev_msp; CUB temporaries bounded
 // above).  count_ctas: resident CTAs of the counting kernel.
 uint64_t bt_job_footprint(uint64_t n, uint64_t m, uint64_t tab_buckets, uint64_t span,
-                          uint64_t count_ctas, bool peel) {
+                          uint64_t count_ctas, uint64_t graphs, bool peel) {
     const uint64_t resident = 36 * m + 16 * n + (1u << 16);
     const uint64_t upload = 32 * m + 52 * n + (16 * m + 24 * n + (4u << 20));
     const uint64_t count = bt_count_bytes(m, span, count_ctas, true) + (1u << 16);
-    const uint64_t msp = peel ? 52 * m + 16 * n + 32 * tab_buckets + (1u << 16) : 0;
+    const uint64_t msp = peel ? 52 * m + 16 * n + 32 * tab_buckets + 2048 * graphs + (1u << 16) : 0;
     return resident + std::max(upload, count + msp);
 }
 
@@ -103,7 +103,7 @@ extern "C" bt_status bt_job_bytes(bt_ctx *ctx, const bt_graph *const *graphs, ui
         tab += tab_buckets_of(graphs[i]);
         span = std::max<uint64_t>(span, graphs[i]->n);
     }
-    *bytes = bt_job_footprint(n, m, tab, span, (uint64_t)dev_count_ctas(ctx), kind_of(op) != 0);
+    *bytes = bt_job_footprint(n, m, tab, span, (uint64_t)dev_count_ctas(ctx), count, kind_of(op) != 0);
     return BT_OK;
 }
 
@@ -131,7 +131,7 @@ struct bt_server {
             tab += r->tab_buckets;
             span = std::max<uint64_t>(span, r->g->n);
         }
-        return bt_job_footprint(n, m, tab, span, count_ctas, kind_of(job[0]->op) != 0);
+        return bt_job_footprint(n, m, tab, span, count_ctas, job.size(), kind_of(job[0]->op) != 0);
     }
 
     // pick a job (lock held); empty if nothing can start now

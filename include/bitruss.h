@@ -158,7 +158,7 @@ double bt_ctx_phase_ms(const bt_ctx *ctx, const char *phase);
  * peel's values, 0 if from the supports; [20..27] SM cycles per CTA of the peeling
  * kernel by step, where the kernel has it: [23] tasks, [26] grid-barrier waits
  * and plans, [27] the rest.  After a batched call, [1] is
- * the sub-rounds summed over its arenas and [7] the number of arenas. */
+ * the sub-rounds summed over its graphs and [7] the number of arenas. */
 bt_status bt_ctx_stats(const bt_ctx *ctx, uint64_t *out, int n);
 
 /* ---- peeling schedule and its autotuner ------------------------------- */

@@ -43,3 +43,27 @@ def test_two_hubs(engine, gpu_ctx, oracle_mod, shared, own):
     res, got_levels = gpu_ctx.msp()
     np.testing.assert_array_equal(res.astype(np.uint64), want)
     assert got_levels == levels
+
+
+# Batches are peeled by teams of CTAs: more graphs than CTAs, fewer, equal ones
+# and very unequal ones, empty ones between; every graph as when peeled alone.
+@pytest.mark.parametrize("sizes", [[40] * 300, [30_000, 50, 50], [2000, 0, 2000, 0, 300], [20_000] + [200] * 60])
+@pytest.mark.parametrize("ctas", [0, 5])
+def test_batches_in_teams(engine, gpu_ctx, sizes, ctas):
+    from gpu_bitruss_gb300 import gen
+    graphs = []
+    for i, m in enumerate(sizes):
+        u, v = gen.er(max(m // 8, 8), max(m // 8, 8), m, seed=i) if m else (np.zeros(0, np.uint32),) * 2
+        graphs.append(engine.Graph.from_edges(u, v))
+    gpu_ctx.set_peel_ctas(ctas)
+    try:
+        for exact in (False, True):
+            res, levels = gpu_ctx.msp_batch(graphs, exact=exact)
+            assert len(res) == len(graphs)
+            for i in {0, 1, len(graphs) // 2, len(graphs) - 1}:
+                gpu_ctx.upload(graphs[i])
+                alone, lv = gpu_ctx.msp(exact=exact)
+                np.testing.assert_array_equal(res[i], alone)
+                assert int(levels[i]) == lv
+    finally:
+        gpu_ctx.set_peel_ctas(0)

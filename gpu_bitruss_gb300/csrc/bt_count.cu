@@ -34,6 +34,10 @@
 //  * Supports are summed per row slot: the slots of a suffix are neighbours, so
 //    32 updates are 4 sectors, where the edge ids' are 32.  k_support adds a
 //    slot's sum to its edge.
+//  * ANY_ORDER (no supports): rows are not sorted, whole rows are walked and ends
+//    that do not rank below the start vertex left out; large vertices take a pass
+//    for each kDense ranks instead of counters in HBM (bt_noalloc.cu has the
+//    figures).
 // Supports of a 2M-edge Chung-Lu graph: 6.6 -> 2.6 ms; of a 4M-edge hub-skewed
 // graph (4e7 wedges, most rows of 10) 7.0 -> 1.1 ms; of a 500k-edge graph of mean
 // degree 8 2.0 -> 0.5 ms.
@@ -100,15 +104,18 @@ __device__ __forceinline__ void acc_add(void *acc, uint32_t slot, unsigned long 
 
 // 32 middle vertices of r, one per lane: where the suffix of ranks above r
 // starts in each one's row, and its length (0 past the end of r's row).
+// ANY_ORDER: rows are not sorted; the whole row of a middle vertex above r is
+// taken, and the visitor leaves out the ranks up to r.
 struct Mid {
     uint32_t p0, len;
 };
+template <bool ANY_ORDER>
 __device__ __forceinline__ Mid load_mid(const CountArgs &a, uint32_t rb, uint32_t rl, uint32_t i, uint32_t r) {
     Mid m{0, 0};
     if (i < rl) {
         const uint32_t s = __ldg(a.nbr + rb + i);
         const uint32_t sb = __ldg(a.off + s), sl = __ldg(a.deg + s);
-        const uint32_t j0 = upper_bound_u32(a.nbr + sb, sl, r);
+        const uint32_t j0 = ANY_ORDER ? (s > r ? 0 : sl) : upper_bound_u32(a.nbr + sb, sl, r);
         m.p0 = sb + j0;
         m.len = sl - j0;
     }
@@ -162,8 +169,9 @@ __device__ __forceinline__ uint32_t light_slot(uint32_t *keys, uint32_t w) {
 
 // All of one small start vertex by one warp (at most kLightWedges wedges);
 // returns the lane's share of the butterflies.  table is zero on entry and exit.
-template <bool PER_EDGE, bool WIDE>
-__device__ __forceinline__ unsigned long long light_vertex(const CountArgs &a, uint32_t *table, uint32_t first,
+template <bool PER_EDGE, bool WIDE, bool ANY_ORDER>
+__device__ __forceinline__ unsigned long long light_vertex(const CountArgs &a, uint32_t *table, uint32_t r,
+                                                           uint32_t first,
                                                            const Mid (&m)[kLightMids / 32], uint32_t total) {
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long local = 0;
@@ -189,6 +197,7 @@ __device__ __forceinline__ unsigned long long light_vertex(const CountArgs &a, u
                 at += cnt;
             });
         }
+        if (ANY_ORDER) have = have && w > r;
         const uint32_t same = __match_any_sync(0xffffffffu, have ? w : 0xffffffffu);
         const uint32_t c = __popc(same);
         if (have && c > 1) {
@@ -203,7 +212,7 @@ __device__ __forceinline__ unsigned long long light_vertex(const CountArgs &a, u
 #pragma unroll
     for (uint32_t q = 0; q < kLightMids / 32; q++)
         visit_wedges(a.nbr, m[q], [&](bool on, uint32_t w, uint32_t, uint32_t) {
-            if (on) local += atomicAdd(cnts + light_slot(keys, w), 1u);
+            if (on && (!ANY_ORDER || w > r)) local += atomicAdd(cnts + light_slot(keys, w), 1u);
         });
     __syncwarp();
     if (PER_EDGE) {
@@ -227,11 +236,12 @@ __device__ __forceinline__ unsigned long long light_vertex(const CountArgs &a, u
 
 // The middle vertices r's row slots [i0, i0 + batch) into sm, those with a
 // suffix only; returns how many.  Starts and ends synchronised.
+template <bool ANY_ORDER>
 __device__ __forceinline__ uint32_t load_batch(const CountArgs &a, CountSmem &sm, uint32_t rb, uint32_t rl,
                                                uint32_t i0, uint32_t r) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t i = i0 + threadIdx.x;
-    const Mid m = load_mid(a, rb, threadIdx.x < a.batch ? rl : 0, i, r);
+    const Mid m = load_mid<ANY_ORDER>(a, rb, threadIdx.x < a.batch ? rl : 0, i, r);
     const uint32_t has = __ballot_sync(0xffffffffu, m.len != 0);
     uint32_t pre = warp_inclusive(m.len);
     if (lane == 31) {
@@ -305,25 +315,28 @@ __device__ __forceinline__ void visit_batch(const uint32_t *nbr, const CountSmem
 
 // All of one large start vertex by the CTA; `dense` is zero on entry and exit.
 // Ends synchronised.
-template <bool PER_EDGE, bool WIDE>
+template <bool PER_EDGE, bool WIDE, bool ANY_ORDER>
 __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, CountSmem &sm, uint32_t *dense,
-                                                         uint32_t r) {
+                                                         uint32_t r, uint32_t skip) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t base = a.seg_base ? a.seg_base[r] : 0u;
     const uint32_t rb = a.off[r], rl = a.deg[r];
-    const uint32_t start = upper_bound_u32(a.nbr + rb, rl, r);
+    const uint32_t start = ANY_ORDER ? 0 : upper_bound_u32(a.nbr + rb, rl, r);
     uint32_t *cnt = a.cnt + (size_t)blockIdx.x * a.span;
     uint32_t *touched = a.touched + (size_t)blockIdx.x * a.span;
-    const uint32_t most = base + a.span - (r + 1);  // ranks of the graph after r
+    // the ranks counted: the first ones of the graph after r and after `skip` more
+    const uint32_t first = r + 1 + skip, most = base + a.span - first;
     const uint32_t near = most < a.dense ? most : a.dense;
     unsigned long long local = 0;
     if (threadIdx.x == 0) sm.touched = 0;
     __syncthreads();
     // pass 1: wedge counts c(r, w) (bfc_vpp.cu:163-187)
     auto count_wedge = [&](uint32_t w) {
-        const uint32_t d = w - (r + 1);
+        const uint32_t d = w - first;
         if (d < near) {
             atomicAdd(dense + d, 1u);
+        } else if (ANY_ORDER) {
+            if (w > r && d - near < 0x80000000u) sm.touched = 1;  // ranks past these: another pass
         } else if (a.span > a.dense && w - base < a.span) {
             const uint32_t old = atomicAdd(cnt + (w - base), 1u);
             local += old;
@@ -336,17 +349,17 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
     auto wedge_share = [&](bool on, uint32_t w) {
         uint32_t c = 0;
         if (on) {
-            const uint32_t d = w - (r + 1);
+            const uint32_t d = w - first;
             if (d < near) c = dense[d];
             else if (a.span > a.dense && w - base < a.span)
                 c = __ldcg(cnt + (w - base));  // written by L2 atomics: bypass L1
         }
         return c > 1 ? c - 1 : 0u;
     };
-    if (rl - start > kBatch && (a.is_u[r] ? a.short_u : a.short_l)) {
+    if (!ANY_ORDER && rl - start > kBatch && (a.is_u[r] ? a.short_u : a.short_l)) {
         // many short suffixes: every warp on its own, 32 of them at a time
         for (uint32_t i0 = start + warp * 32; i0 < rl; i0 += kBatch)
-            visit_wedges(a.nbr, load_mid(a, rb, rl, i0 + lane, r), [&](bool on, uint32_t w, uint32_t, uint32_t) {
+            visit_wedges(a.nbr, load_mid<ANY_ORDER>(a, rb, rl, i0 + lane, r), [&](bool on, uint32_t w, uint32_t, uint32_t) {
                 if (on) count_wedge(w);
             });
         __syncthreads();
@@ -355,7 +368,7 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
             for (uint32_t i0 = start + warp * 32; i0 < rl; i0 += kBatch) {
                 sum[lane] = 0;
                 __syncwarp();
-                visit_wedges(a.nbr, load_mid(a, rb, rl, i0 + lane, r), [&](bool on, uint32_t w, uint32_t p, uint32_t k) {
+                visit_wedges(a.nbr, load_mid<ANY_ORDER>(a, rb, rl, i0 + lane, r), [&](bool on, uint32_t w, uint32_t p, uint32_t k) {
                     const uint32_t add = wedge_share(on, w);
                     if (!add) return;
                     acc_add<WIDE>(a.acc, p, add);
@@ -372,7 +385,7 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
     } else {
         uint32_t nm = 0;
         for (uint32_t i0 = start; i0 < rl; i0 += a.batch) {
-            nm = load_batch(a, sm, rb, rl, i0, r);
+            nm = load_batch<ANY_ORDER>(a, sm, rb, rl, i0, r);
             visit_batch(a.nbr, sm, nm, [&](bool on, uint32_t w, uint32_t, uint32_t, bool) {
                 if (on) count_wedge(w);
             });
@@ -380,7 +393,7 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
         }
         // a single batch is still loaded
         for (uint32_t i0 = start; PER_EDGE && i0 < rl; i0 += a.batch) {
-            if (rl - start > a.batch) nm = load_batch(a, sm, rb, rl, i0, r);
+            if (rl - start > a.batch) nm = load_batch<ANY_ORDER>(a, sm, rb, rl, i0, r);
             visit_batch(a.nbr, sm, nm, [&](bool on, uint32_t w, uint32_t p, uint32_t k, bool uniform) {
                 const uint32_t add = wedge_share(on, w);
                 if (add) acc_add<WIDE>(a.acc, p, add);
@@ -413,18 +426,21 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
             d4[k] = make_uint4(0, 0, 0, 0);
         }
     }
-    const uint32_t nt = sm.touched;
-    for (uint32_t k = threadIdx.x; k < nt; k += kCountThreads) cnt[touched[k]] = 0;
+    if constexpr (!ANY_ORDER) {
+        const uint32_t nt = sm.touched;
+        for (uint32_t k = threadIdx.x; k < nt; k += kCountThreads) cnt[touched[k]] = 0;
+    }
     __syncthreads();
     return local;
 }
 
-template <bool PER_EDGE, bool WIDE>
-__global__ void __launch_bounds__(kCountThreads) k_count(const __grid_constant__ CountArgs a) {
+template <bool PER_EDGE, bool WIDE, bool ANY_ORDER>
+__global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constant__ CountArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CountSmem &sm = *reinterpret_cast<CountSmem *>(smem_raw);
     uint32_t *dense = reinterpret_cast<uint32_t *>(smem_raw + sizeof(CountSmem));  // also the warps' hashes
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (ANY_ORDER && *a.layout_error) return;  // nothing to count here: see bt_count_any_order
     const uint32_t words = a.dense > kCountWarps * 2 * kSlots ? a.dense : kCountWarps * 2 * kSlots;
     for (uint32_t k = threadIdx.x; k < words; k += kCountThreads) dense[k] = 0;
     __syncthreads();
@@ -437,7 +453,7 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const __grid_constant__
         if (r < a.n) {
             const uint32_t rb = __ldg(a.off + r), rl = __ldg(a.deg + r);
             // the suffix of r's own row after r, found 32 ways at a time
-            uint32_t lo = 0, hi = rl;
+            uint32_t lo = 0, hi = ANY_ORDER ? 0 : rl;
             while (hi > lo) {
                 const uint32_t step = (hi - lo + 31) / 32, i = lo + lane * step;
                 const uint32_t le = __popc(__ballot_sync(0xffffffffu, i < hi && __ldg(a.nbr + rb + i) <= r));
@@ -457,20 +473,30 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const __grid_constant__
                 uint32_t sum = 0;
 #pragma unroll
                 for (uint32_t q = 0; q < kLightMids / 32; q++) {
-                    m[q] = load_mid(a, rb, rl, lo + q * 32 + lane, r);
+                    m[q] = load_mid<ANY_ORDER>(a, rb, rl, lo + q * 32 + lane, r);
                     sum += min(m[q].len, kLightWedges + 1);
                 }
                 const uint32_t total = __reduce_add_sync(0xffffffffu, sum);
                 if (total > kLightWedges) big = r + 1;
-                else if (total) local += light_vertex<PER_EDGE, WIDE>(a, table, rb + lo, m, total);
+                else if (total) local += light_vertex<PER_EDGE, WIDE, ANY_ORDER>(a, table, r, rb + lo, m, total);
             }
         }
         if (lane == 0) sm.big[warp] = big;
         if (threadIdx.x == 0) sm.chunk = gridDim.x + atomicAdd(a.next_chunk, 1u);
         __syncthreads();
         c = sm.chunk;
-        for (uint32_t w = 0; w < kCountWarps; w++)
-            if (sm.big[w]) local += big_vertex<PER_EDGE, WIDE>(a, sm, dense, sm.big[w] - 1);
+        for (uint32_t w = 0; w < kCountWarps; w++) {
+            if (!sm.big[w]) continue;
+            const uint32_t v = sm.big[w] - 1;
+            bool more;
+            uint32_t skip = 0;
+            do {  // no counters but the shared ones: further passes over the ranks past them
+                local += big_vertex<PER_EDGE, WIDE, ANY_ORDER>(a, sm, dense, v, skip);
+                more = ANY_ORDER && sm.touched != 0;
+                if (ANY_ORDER) __syncthreads();
+                skip += a.dense;
+            } while (more);
+        }
         __syncthreads();
     }
     for (int o = 16; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
@@ -512,8 +538,8 @@ size_t count_smem(uint32_t dense) {
 }
 
 const void *count_kernel(bool per_edge, bool wide) {
-    if (!per_edge) return (const void *)k_count<false, false>;
-    return wide ? (const void *)k_count<true, true> : (const void *)k_count<true, false>;
+    if (!per_edge) return (const void *)k_count<false, false, false>;
+    return wide ? (const void *)k_count<true, true, false> : (const void *)k_count<true, false, false>;
 }
 
 }  // namespace
@@ -606,5 +632,32 @@ bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count) {
         ctx->last_result = 1;
     }
     ctx->last_count = h[0];
+    return BT_OK;
+}
+
+static const void *any_order_kernel() { return (const void *)k_count<false, false, true>; }
+
+bt_status bt_count_any_order_setup() {
+    BT_CUDA(cudaFuncSetAttribute(any_order_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)count_smem(kDense)));
+    return BT_OK;
+}
+
+bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *deg, const uint32_t *nbr,
+                             unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st) {
+    CountArgs a{};
+    a.n = a.span = n;
+    a.dense = dense_of(n);
+    a.chunks = (n + kCountWarps - 1) / kCountWarps;
+    a.batch = (uint32_t)std::min<uint64_t>(kBatch, 0xffffffffull / n);  // degrees are below n
+    a.off = off;
+    a.deg = deg;
+    a.nbr = nbr;
+    a.count = count;
+    a.next_chunk = next_chunk;
+    a.layout_error = skip;
+    void *params[] = {&a};
+    BT_CUDA(cudaLaunchKernel(any_order_kernel(), dim3(std::min<uint32_t>((uint32_t)sms, a.chunks)), dim3(kCountThreads),
+                             params, count_smem(a.dense), st));
+    bt_note_launches(1);
     return BT_OK;
 }

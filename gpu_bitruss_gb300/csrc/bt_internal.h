@@ -163,6 +163,15 @@ void ctx_release_graph(bt_ctx *ctx);
 // most bytes the counting kernel's scratch takes (bt_count.cu)
 uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide);
 
+// Butterflies of one graph given by ranks, its rows in any order, on one CTA per
+// SM with counters in shared memory only; every buffer is the caller's and
+// nothing is allocated.  Degrees are below n, n < 2^31.  *next_chunk is zero on
+// entry; nothing is counted if *skip is not (bt_count.cu).  The set-up is made
+// once per device and context.
+bt_status bt_count_any_order_setup();
+bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *deg, const uint32_t *nbr,
+                             unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st);
+
 // algorithm entry points implemented in the .cu files
 bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *g);
 bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count);

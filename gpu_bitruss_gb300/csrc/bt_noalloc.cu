@@ -17,20 +17,20 @@
 //    shared memory and runs on every SM; each 52k vertices past the first cost
 //    the large start vertices one more pass over their wedges.  For graphs that
 //    fit, of at least kRankEdges edges: six kernels in a row take 40 us, so below
-//    them the other way is as fast (16k edges: 43-54 us by ranks, 33-61 us by
-//    counters; 32k: 47 and 55 us).
+//    them the other way is as fast (16k edges: 44-53 us by ranks, 33-61 us by
+//    counters; 25k: 49-55 and 44-88 us).
 //  * Counters.  Each CTA uses 2n words (a wedge counter and a touched list per
 //    vertex), so the count runs on min(2 per SM, kScratchWords / 2n) CTAs; every
 //    priority test reads two row offsets.  Also for what the ranks' kernels find
 //    on the way to be no graph in the layout (below): a flag on the device
 //    chooses, no host read.
-// Measured, by counters and by ranks: 300k edges on 69k vertices (skewed) 1,822
-// and 271 us; 300k on 176k vertices 9,600 and 339 us; 1M on 140k 9,918 and 1,097
-// us; 1M on 641k 117,028 and 1,348 us.  By counters the bound is the few CTAs
-// that the scratch has room for (60 at 69k vertices, 6 at 641k) and two offset
-// loads per wedge; by ranks it is the wedges' shared-memory atomics.
 // Graphs of more than kScratchWords / 2 vertices are rejected.  The last 64
 // words hold the work counters and the flag.
+// Measured, by counters and by ranks: 300k edges on 69k vertices (skewed) 1,822
+// and 243 us; 300k on 176k vertices 9,600 and 282 us; 1M on 140k 9,918 and 1,037
+// us; 1M on 641k 117,028 and 1,142 us.  By counters the bound is the few CTAs
+// that the scratch has room for (60 at 69k vertices, 6 at 641k) and two offset
+// loads per wedge; by ranks it is the wedges' shared-memory atomics.
 //
 // All calls share the array: calls that overlap on the GPU (on different
 // streams or threads, without ordering between them) race on it and give
@@ -58,7 +58,7 @@
 #include <mutex>
 #include <string>
 
-#include "bt_internal.h"
+#include "bt_device.cuh"
 
 namespace {
 
@@ -182,7 +182,9 @@ __global__ void k_na_degrees(uint32_t n, uint64_t m, const uint32_t *off, Ranks 
     for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
         const uint32_t d = off[x + 1] - off[x];
         if (d < n) {
-            atomicAdd(t.bins + d, 1u);
+            // the lanes of one degree add together: most vertices share a few
+            const uint32_t same = __match_any_sync(__activemask(), d);
+            if ((threadIdx.x & 31) == (uint32_t)__ffs(same) - 1) atomicAdd(t.bins + d, (uint32_t)__popc(same));
             most = d > most ? d : most;
         } else {
             bad = true;
@@ -248,21 +250,18 @@ __global__ void k_na_rank(uint32_t n, const uint32_t *off, Ranks t, const Words 
     }
 }
 
-// The rows with ranks in place of vertices; one warp per vertex.  Rows that do
-// not ascend strictly may hold a neighbour twice: then the order of equal
+// The rows with ranks in place of vertices; one thread per slot (a warp per row
+// waits for the longest: 100 us of the 300k-edge graph's 314, now 15).  Rows that
+// do not ascend strictly may hold a neighbour twice: then the order of equal
 // degrees matters to the count, and the other way keeps it by vertex id.
-__global__ void k_na_rows(uint32_t n, const uint32_t *off, const uint32_t *nbr, Ranks t, Words *w) {
+__global__ void k_na_rows(uint32_t n, const uint32_t *off, const uint32_t *nbr, uint64_t slots, Ranks t, Words *w) {
     if (w->irregular) return;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     bool bad = false;
-    for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < n; x += nw) {
-        const uint32_t b = off[x], d = off[x + 1] - b, dst = t.off[t.rank[x]];
-        for (uint32_t j = lane; j < d; j += 32) {
-            const uint32_t y = nbr[b + j];
-            if (y >= n || (j && nbr[b + j - 1] >= y)) bad = true;
-            t.nbr[dst + j] = y < n ? t.rank[y] : 0;
-        }
+    for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < slots; p += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t y = nbr[p], before = p ? nbr[p - 1] : 0;
+        const uint32_t x = bt::row_of_slot(off, n, (uint32_t)p), j = (uint32_t)p - off[x];
+        if (y >= n || (j && before >= y)) bad = true;
+        t.nbr[t.off[t.rank[x]] + j] = y < n ? t.rank[y] : 0;
     }
     if (bad) w->irregular = 1;
 }
@@ -322,11 +321,12 @@ extern "C" bt_status bt_bfc_noalloc(int device, const uint32_t *d_offsets, const
         uint32_t *p = scratch;
         const Ranks t{p, p + n, p + 2ull * n, p + 3ull * n, p + 4ull * n, p + 5ull * n, p + 6ull * n};
         BT_CUDA(cudaMemsetAsync(t.bins, 0, 8ull * n, st));  // and taken
-        const unsigned most = (unsigned)sms * 8, per_vertex = std::min(most, (n + 255) / 256), per_row = std::min(most, (n + 7) / 8);
+        const unsigned most = (unsigned)sms * 8, per_vertex = std::min(most, (n + 255) / 256);
+        const unsigned per_slot = (unsigned)std::min<uint64_t>(most, (2 * m + 255) / 256);
         k_na_degrees<<<per_vertex, 256, 0, st>>>(n, m, d_offsets, t, words);
         k_na_scan<<<1, 1024, 0, st>>>(t, words);
         k_na_rank<<<per_vertex, 256, 0, st>>>(n, d_offsets, t, words);
-        k_na_rows<<<per_row, 256, 0, st>>>(n, d_offsets, d_neighbors, t, words);
+        k_na_rows<<<per_slot, 256, 0, st>>>(n, d_offsets, d_neighbors, 2 * m, t, words);
         bt_note_launches(4);
         BT_CUDA(cudaGetLastError());
         BT_TRY(bt_count_any_order(n, t.off, t.deg, t.nbr, d_count, &words->next_chunk, &words->irregular, sms, st));

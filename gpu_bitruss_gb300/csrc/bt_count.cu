@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (ANY_ORDER && *a.layout_error) return;  // nothing to count here: see bt_count_any_order
     const uint32_t words = a.dense > kCountWarps * 2 * kSlots ? a.dense : kCountWarps * 2 * kSlots;
-    for (uint32_t k = threadIdx.x; k < words; k += kCountThreads) dense[k] = 0;
+    uint4 *d4 = reinterpret_cast<uint4 *>(dense);
+    for (uint32_t k = threadIdx.x; k < words / 4; k += kCountThreads) d4[k] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     uint32_t *table = dense + warp * 2 * kSlots;
     unsigned long long local = 0;
@@ -619,8 +620,11 @@ bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count) {
         }
     }
     cudaEventRecord(ctx->ev[7], st);
-    uint64_t h[4] = {0, 0, 0, 0};
-    BT_CUDA(cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st));
+    // one wait for the kernels, the results and the callers' end time: a staged
+    // copy and a second wait cost a 20k-edge count 9 of its 51 us
+    const uint64_t *h = ctx->host_words;
+    BT_CUDA(cudaMemcpyAsync(ctx->host_words, head, 32, cudaMemcpyDeviceToHost, st));
+    cudaEventRecord(ctx->ev[1], st);
     BT_CUDA(cudaStreamSynchronize(st));
     if ((uint32_t)h[3]) return bt_fail(BT_ERR_INVALID, "butterfly count: a wedge left its graph in the arena layout");
     ctx->zero_counters = far;

@@ -177,6 +177,12 @@ extern "C" bt_status bt_ctx_create(int device, bt_ctx **out) {
         return bt_cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
     ctx->stream = ctx->own_stream;
+    e = cudaHostAlloc((void **)&ctx->host_words, 4 * sizeof(uint64_t), cudaHostAllocDefault);
+    if (e != cudaSuccess) {
+        cudaStreamDestroy(ctx->own_stream);
+        delete ctx;
+        return bt_cuda_fail(e, "cudaHostAlloc", __FILE__, __LINE__);
+    }
     for (auto &ev : ctx->ev) cudaEventCreate(&ev);
     pool_setup(device);
     *out = ctx;
@@ -218,6 +224,7 @@ extern "C" void bt_ctx_free(bt_ctx *ctx) {
     cudaStreamSynchronize(ctx->own_stream);
     for (auto &ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
+    cudaFreeHost(ctx->host_words);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
 }
@@ -497,6 +504,11 @@ static bt_status need_graph(bt_ctx *ctx) {
 }
 
 static void time_begin(bt_ctx *ctx) { cudaEventRecord(ctx->ev[0], ctx->stream); }
+// dev_ebfc has recorded the end and waited for it
+static void time_counted(bt_ctx *ctx, int phase) {
+    float ms = -1;
+    if (cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]) == cudaSuccess) ctx->phase_ms[phase] = ms;
+}
 static void time_end(bt_ctx *ctx, int phase) {
     cudaEventRecord(ctx->ev[1], ctx->stream);
     cudaEventSynchronize(ctx->ev[1]);
@@ -527,7 +539,7 @@ extern "C" bt_status bt_bfc(bt_ctx *ctx, uint64_t *count) {
     time_begin(ctx);
     uint64_t c = 0;
     BT_TRY(dev_ebfc(ctx, false, &c));
-    time_end(ctx, PH_TOTAL);
+    time_counted(ctx, PH_TOTAL);
     if (count) *count = c;
     return BT_OK;
 }
@@ -538,7 +550,7 @@ extern "C" bt_status bt_ebfc(bt_ctx *ctx, uint64_t *sup, uint64_t *count, uint64
     time_begin(ctx);
     uint64_t c = 0;
     BT_TRY(dev_ebfc(ctx, true, &c));
-    time_end(ctx, PH_TOTAL);
+    time_counted(ctx, PH_TOTAL);
     if (count) *count = c;
     if (support_max) *support_max = ctx->last_sup_max;
     return copy_out(ctx, sup, ctx->sup, 8 * ctx->g.m);

@@ -135,6 +135,7 @@ struct bt_ctx {
     uint64_t work[12] = {0};  // msp work counters and phase times of the last call
     uint64_t prof[8] = {0};   // msp: SM cycles per CTA by step (task, stage, slice, probe, hits, flush, barrier, other)
     cudaEvent_t ev[8] = {};
+    uint64_t *host_words = nullptr;  // 4 page-locked words: a count's results come back without a staging copy
 
     // msp task schedule (0 = built-in value): positions per task, chunks per CTA, whole-plan limit
     uint32_t msp_schedule[3] = {0, 0, 0};

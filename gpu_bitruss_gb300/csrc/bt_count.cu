@@ -565,7 +565,9 @@ bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count) {
     const void *kfn = count_kernel(per_edge, wide);
     const size_t smem = count_smem(dense);
     const uint32_t chunks = (g.n + kCountWarps - 1) / kCountWarps;
-    BT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit belongs to the kernel, not to the call: the same value from every
+    // thread, or one with a smaller graph lowers it before another's launch
+    BT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)count_smem(kDense)));
     // one CTA per SM (its counters fill the SM's shared memory)
     const uint64_t nctas = std::max<uint64_t>(1, std::min<uint64_t>(ctx->sm_count, chunks));
     // scratch: [0, 64) count, support max, work counter, layout error; then the

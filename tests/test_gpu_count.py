@@ -54,3 +54,29 @@ def test_wide_sums(engine, gpu_ctx, oracle_mod):
     u = np.concatenate([np.zeros(k, np.int64), np.arange(1, k), np.repeat(np.arange(1, 4), 500)])
     v = np.concatenate([np.arange(k), np.zeros(k - 1, np.int64), np.tile(np.arange(1, 501), 3)])
     _check(engine, gpu_ctx, oracle_mod, u, v)
+
+
+def test_small_and_large_side_by_side(engine, oracle_mod):
+    """Contexts of several threads count graphs that want different amounts of
+    shared memory, over and over, at the same time."""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(7)
+
+    def count(n):
+        u, v = rng_edges[n]
+        want = oracle_mod.ebfc(oracle_mod.build_csr(u, v), 0)[1]
+        ctx = engine.Context(0)
+        try:
+            ctx.upload(engine.Graph.from_edges(u, v))
+            return [ctx.bfc() for _ in range(300)], want
+        finally:
+            ctx.close()
+
+    sizes = (1000, 40_000, 60_000, 90_000)
+    rng_edges = {}
+    for n in sizes:
+        key = np.unique(rng.integers(0, n // 2, 2 * n) * n + rng.integers(0, n // 2, 2 * n))
+        rng_edges[n] = ((key // n).astype(np.uint32), (key % n).astype(np.uint32))
+    with ThreadPoolExecutor(len(sizes)) as pool:
+        for got, want in pool.map(count, sizes):
+            assert got == [want] * 300

@@ -98,9 +98,9 @@ def load_peaks():
 
 # DRAM bytes per k_msp launch, measured by ncu on graphs larger than L2 but
 # small enough to capture (profiles/k_msp_dram_traffic.md).  The traffic per
-# row position grows with the graph (2M edges: 1.17 B, 5M: 10.57 B), so it is
+# row position grows with the graph (2M edges: 0.09 B, 5M: 1.21 B), so it is
 # not scaled to other sizes: other workloads report none.
-DRAM_TRAFFIC = {"cl2000k": 14_827_734_272 + 2_185_049_344, "cl5000k": 608_334_618_112 + 70_095_516_672}
+DRAM_TRAFFIC = {"cl2000k": 1_038_540_288 + 322_856_192, "cl5000k": 70_263_388_160 + 7_102_622_208}
 
 
 def load_traffic(workload):
@@ -344,9 +344,8 @@ def run_ours(args):
                    "step_wall_ms": statistics.median(walls), "gen_s": round(t_gen, 1),
                    "schedule": list(ctx.msp_schedule()),
                    "kernel_phase_ms": {"level_transitions": work[6] / 1e6, "peel": work[7] / 1e6},
-                   "cta_ms_by_step": dict(zip(["task", "stage", "slice", "probe", "hits", "flush",
-                                               "barrier", "other"],
-                                              [round(c / (mhz * 1e3), 1) for c in stats[20:28]]))},
+                   "cta_ms_by_step": {k: round(stats[20 + i] / (mhz * 1e3), 1)
+                                      for k, i in (("probe", 3), ("barrier", 6), ("other", 7))}},
         "e2e": {"value": e2e_value, "unit": "edges/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h),
                 "note": "every step: CSR from pageable host memory, bt_msp, bitruss numbers to host"},

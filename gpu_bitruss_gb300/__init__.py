@@ -361,8 +361,7 @@ class Context:
         butterflies found, decrements, m, ns in level transitions, ns in
         peel phases, ns in finalize phases, bytes per working support (4 or 8),
         -, -, then SM cycles per CTA
-        of the peeling kernel by step: task, stage, slice, probe, hits, flush,
-        barrier, other]"""
+        of the peeling kernel by step: -, -, -, probe, -, -, barrier, other]"""
         a = (C.c_uint64 * 28)()
         _check(load().bt_ctx_stats(self._c, a, 28), "stats")
         return list(a)

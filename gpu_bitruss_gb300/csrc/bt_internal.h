@@ -133,7 +133,7 @@ struct bt_ctx {
     double phase_ms[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
     uint64_t stats[8] = {0};
     uint64_t work[12] = {0};  // msp work counters and phase times of the last call
-    uint64_t prof[8] = {0};   // msp: SM cycles per CTA by step (task, stage, slice, probe, hits, flush, barrier, other)
+    uint64_t prof[8] = {0};   // msp: SM cycles per CTA by step (3 walking, 6 at barriers, 7 the rest)
     cudaEvent_t ev[8] = {};
     uint64_t *host_words = nullptr;  // 4 page-locked words: a count's results come back without a staging copy
 

@@ -15,13 +15,13 @@
 //
 // Continuous batching: when a slot takes a request, every queued request of
 // the same kind (supports/counts, msp, exact msp) that also fits joins it, up
-// to kBatchEdges edges; requests above kSoloEdges edges run alone.  Together they form one arena (bt_graph_pack layout),
-// uploaded once and run by one launch sequence.  A request's result is the
+// to kBatchEdges edges; requests above kSoloEdges edges run alone.  Together they
+// form one arena (bt_graph_pack layout), uploaded once and run by one launch sequence.  A request's result is the
 // same alone and in a batch: butterflies never span two graphs of an arena.
 //
-// One cooperative peeling kernel runs at a time in the process (dev_msp
-// serialises them); counting kernels, uploads and copies of other slots run
-// beside it.
+// The slots' peels run side by side on shares of the SMs (CtaSlots in bt_msp.cu
+// keeps their cooperative grids resident together); counting kernels, uploads
+// and copies of other slots run beside them.
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>

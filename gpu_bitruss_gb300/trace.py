@@ -2,7 +2,7 @@
 
 Setting ``BT_MSP_TRACE=<path>`` makes ``bt_msp`` write one record per
 sub-round: the sub-round's duration as seen by CTA 0 (plan to barrier exit),
-its longest task, the row positions walked, the frontier size and the task
+its longest CTA's part, the row positions walked, the frontier size and the task
 count.  Usage::
 
     BT_MSP_TRACE=trace.bin python bench.py --steps 1 --warmup 0 --no-cpu

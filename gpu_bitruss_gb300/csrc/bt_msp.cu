@@ -99,15 +99,39 @@ constexpr uint32_t kWarps = kThreads / 32;
 constexpr uint32_t kEdges = kMspLocalPlan;  // frontier edges a CTA plans at once
 
 // What every CTA reads after a barrier, in one warp-wide load (barrier()).
+//
+// A CTA that leaves a barrier first goes on while others have yet to load these
+// words.  So no word that a CTA uses after barrier b may be written between b
+// and the barrier after it.  For each word, who writes it, and the barrier
+// (S: a level's scan, P: a sub-round, F1 / F2: the two of a far split) after
+// which it is used:
+//  * len[r % 3]: appended to by sub-round r - 1 only, used after its P; zeroed in
+//    sub-round r + 1.
+//  * scan_len[k % 3]: appended to by the scan of level number k only, used after
+//    that S (and after the barriers of a row compaction behind it); zeroed at the
+//    scan of number k + 2.  It is not len: a CTA that finds len at 0 after a P goes
+//    straight to the scan, as a slower one must, which reads the same len.
+//  * cand[k % 3]: lowered at the S of level number k and at its P's, used when that
+//    level has run out: after its last P, or S if it was empty; reset at the
+//    scan of number k + 2.
+//  * near_ctr[nsel]: appended to by sub-rounds, used at a scan, after the last P,
+//    F2 or S.  near_ctr[nsel ^ 1]: appended to between F1 and F2 or by a scan that
+//    compacts, used after that F2 or S as the new near_ctr[nsel]; the one left is
+//    zeroed behind the same barrier and next appended to behind another (near_dead
+//    is 0 there, so a scan that follows at once does not compact).
+//  * far_len, far2_len, far_min, delta: far2_len is appended to and far_min
+//    lowered before F2 and F1, and used after them; all four are set behind
+//    F2 and next used after the S that follows at the earliest.
 struct Control {
     unsigned long long delta;      // width of the near bucket
     unsigned long long far_min;
     // cand[k % 3]: a lower bound of the supports that are live above level
     // number k, collected while that level is scanned and peeled
     unsigned long long cand[3];
-    uint32_t len[3];               // frontier list lengths by sub-round index mod 3
+    uint32_t len[3];               // lengths of the frontiers that sub-rounds find, by index mod 3
+    uint32_t scan_len[3];          // of those that levels' scans find, by level number mod 3
     uint32_t near_ctr[2];          // near bucket lengths (selector kept by every CTA)
-    uint32_t far_len, far2_len, pad;
+    uint32_t far_len, far2_len;
 };
 constexpr uint32_t kControlWords = sizeof(Control) / 4;
 static_assert(kControlWords <= 32, "the control words are loaded by one warp");
@@ -187,6 +211,7 @@ struct MspArgs {
     float inv_task;                 // 1 / positions of a task
     uint64_t m;
     unsigned long long wait_ns;
+    uint32_t late_ns;               // see linger()
     const uint2 *ends;
     VRec *vrec;
     uint32_t *nbr, *eid;            // live rows (compacted in place)
@@ -449,11 +474,18 @@ __device__ __forceinline__ void plan_block(const MspArgs &a, Smem &sm, const uin
     __syncthreads();
 }
 
+// BT_MSP_LATE_NS: an eighth of the CTAs, other ones each time, stay about that
+// long between a barrier and what they read behind it.  Whatever the others do
+// meanwhile, the results are the same.
+__device__ __forceinline__ void linger(const MspArgs &a, uint32_t epoch) {
+    if (a.late_ns && ((blockIdx.x * 0x9E3779B1u ^ epoch * 0x85EBCA6Bu) * 0xC2B2AE35u >> 29) == 0) __nanosleep(a.late_ns);
+}
+
 // Barrier of the team.  Publishes the CTA's running minimum to cand[k3], refreshes
-// sm.now, and with `plan` plans the next frontier (length len[r3], list `list`)
-// when it is a short one: its entries come with the control words.
-__device__ __forceinline__ bool barrier(const MspArgs &a, const Team &t, Smem &sm, uint32_t &epoch, uint32_t k3, uint32_t r3,
-                                        uint32_t list, bool plan) {
+// sm.now, and with `plan` plans the next frontier (`len`, a word of sm.now, is its length,
+// `list` its list) when it is a short one: its entries come with the control words.
+__device__ __forceinline__ bool barrier(const MspArgs &a, const Team &t, Smem &sm, uint32_t &epoch, uint32_t k3,
+                                        const uint32_t &len, uint32_t list, bool plan) {
     __syncthreads();
     prof_mark(sm, PF_OTHER);
     int ok = 1;
@@ -469,11 +501,12 @@ __device__ __forceinline__ bool barrier(const MspArgs &a, const Team &t, Smem &s
         epoch += t.size;
         ok = bt::barrier_wait(t.bar, epoch, a.wait_ns);
         if (!ok) a.sh->error = bt::ERR_TIMEOUT;
+        linger(a, epoch);
         const uint4 head = load_control(t.s, sm, list);
         __syncwarp();
-        const uint32_t len = sm.now.len[r3];
-        if (plan && len - 1 < 32 && len <= a.local_plan)
-            plan_warp(a, sm, len, head, t.size * kWarps, t.rank == 0);
+        const uint32_t cnt = len;
+        if (plan && cnt - 1 < 32 && cnt <= a.local_plan)
+            plan_warp(a, sm, cnt, head, t.size * kWarps, t.rank == 0);
     }
     ok = __syncthreads_and(ok);
     prof_mark(sm, PF_BARRIER);
@@ -743,6 +776,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
             epoch += t.size;
             ok = bt::barrier_wait(t.bar, epoch, a.wait_ns);
             if (!ok) a.sh->error = bt::ERR_TIMEOUT;
+            linger(a, epoch);
             const uint32_t q = __ldcg(&team->job);
             if (threadIdx.x == 0) sm.chunk = q;
             if (q < a.njobs) load_control(a.states + q, sm, 0);
@@ -764,7 +798,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
         unsigned long long live = sm.now.far_len, live_at_compress = t.job.m;
         for (;;) {
             // ------------------------------------------------ level transition
-            if (sm.now.len[r3] == 0) {
+            uint32_t curr_len = sm.now.len[r3];
+            if (curr_len == 0) {
                 bool squeeze = false, dry = false;
                 for (;;) {
                     L = sm.now.cand[k3];
@@ -772,7 +807,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                         // near is dry: split the far bucket
                         const uint32_t far_len = sm.now.far_len;
                         list_min<N32>(a, t, far0, far_len, &s->ctl.far_min);
-                        if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                        if (!barrier(a, t, sm, epoch, k3, sm.now.len[r3], r & 1, false)) return;
                         L = sm.now.far_min;
                         if (L == ~0ull) {  // nothing left
                             dry = true;
@@ -786,7 +821,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                             if (sup_of<N32>(a, e) < hi) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
                             else far1[atomicAdd(&s->ctl.far2_len, 1u)] = e;
                         }
-                        if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                        if (!barrier(a, t, sm, epoch, k3, sm.now.len[r3], r & 1, false)) return;
                         {   // every CTA swaps its copies of the bucket pointers
                             uint32_t *t = near0; near0 = near1; near1 = t;
                             t = far0; far0 = far1; far1 = t;
@@ -794,7 +829,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                         nsel ^= 1;
                         near_dead = 0;
                         if (clerk) {
-                            // read again after the next barrier at the earliest
                             s->ctl.near_ctr[nsel ^ 1] = 0;
                             s->ctl.far_len = sm.now.far2_len;
                             s->ctl.far2_len = 0;
@@ -809,7 +843,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                     // the lowest support above it; entries processed meanwhile are
                     // dropped from the list once they are half of it
                     k3 = next3(k3);
-                    if (clerk) s->ctl.cand[next3(k3)] = ~0ull;
+                    if (clerk) {
+                        s->ctl.cand[next3(k3)] = ~0ull;
+                        s->ctl.scan_len[next3(k3)] = 0;
+                    }
                     const uint32_t near_len = sm.now.near_ctr[nsel];
                     const bool compact = near_len > gsz && near_dead > near_len / 2;
                     uint32_t *front = ((r & 1 ? a.list1 : a.list0) + e0);
@@ -820,7 +857,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                         const SupWord<N32> v = sup_of<N32>(a, e);
                         if (en != 0) continue;
                         if (v == L) {
-                            list_append(a, front, &s->ctl.len[r3], s->head[r & 1], e, 0, 0, 1, r, (uint32_t)L);
+                            list_append(a, front, &s->ctl.scan_len[k3], s->head[r & 1], e, 0, 0, 1, r, (uint32_t)L);
                         } else {
                             if (v < low) low = v;
                             if (compact) near1[atomicAdd(&s->ctl.near_ctr[nsel ^ 1], 1u)] = e;
@@ -829,7 +866,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                     fold_low<N32>(sm, low);
                     squeeze = (double)live <= (double)a.cfrac * (double)live_at_compress &&
                               (double)live_at_compress >= (double)a.cfloor * (double)t.job.m;
-                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, true)) return;
+                    if (!barrier(a, t, sm, epoch, k3, sm.now.scan_len[k3], r & 1, true)) return;
+                    curr_len = sm.now.scan_len[k3];
                     if (compact) {
                         uint32_t *t = near0; near0 = near1; near1 = t;
                         nsel ^= 1;
@@ -838,7 +876,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                     }
                     // no edge at L: the minimum was of an edge that has since left;
                     // what this scan collected is exact
-                    if (sm.now.len[r3] != 0) break;
+                    if (curr_len != 0) break;
                 }
                 if (dry) break;
                 if (clerk) {
@@ -850,9 +888,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                     live_at_compress = live;
                     if (clerk) compressions++;
                     compress_rows(a, t, r);
-                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, false)) return;
+                    if (!barrier(a, t, sm, epoch, k3, sm.now.scan_len[k3], r & 1, false)) return;
                     prepare_rows(a, t);
-                    if (!barrier(a, t, sm, epoch, k3, r3, r & 1, true)) return;
+                    if (!barrier(a, t, sm, epoch, k3, sm.now.scan_len[k3], r & 1, true)) return;
                 }
                 if (clerk) {
                     const unsigned long long t = clock64();
@@ -861,7 +899,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                 }
             }
             // ------------------------------------------------ sub-round r
-            const uint32_t curr_len = sm.now.len[r3];
             Round<N32> rd;
             rd.r = r;
             rd.L = (SupWord<N32>)L;
@@ -895,7 +932,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                 }
                 if (threadIdx.x == 0) atomicAdd(&a.trace[r].tasks, (uint32_t)(sm.tasks - tasks0));
             }
-            if (!barrier(a, t, sm, epoch, k3, next3(r3), (r + 1) & 1, true)) return;
+            if (!barrier(a, t, sm, epoch, k3, sm.now.len[next3(r3)], (r + 1) & 1, true)) return;
             if (clerk) {
                 const unsigned long long t = clock64();
                 if (a.trace && r < a.trace_cap) {
@@ -1108,6 +1145,11 @@ static unsigned long long wait_limit_ns() {
     return ms * 1000000ull;
 }
 
+static uint32_t late_ns() {
+    const char *v = getenv("BT_MSP_LATE_NS");
+    return v ? (uint32_t)std::min<unsigned long long>(strtoull(v, nullptr, 10), 1000000ull) : 0u;
+}
+
 static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     uint64_t dummy = 0;
     BT_TRY(dev_ebfc(ctx, true, &dummy));
@@ -1221,6 +1263,7 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     a.chunks_per_cta = ctx->msp_schedule[1] ? ctx->msp_schedule[1] : kMspTasksPerCta;
     a.local_plan = std::min(ctx->msp_schedule[2] ? ctx->msp_schedule[2] : kMspLocalPlan, kEdges);
     a.wait_ns = wait_limit_ns();
+    a.late_ns = late_ns();
     // Row compaction: whenever the live edges have halved since the last
     // compaction.  The reference also stops compacting once fewer than a tenth
     // of all edges are live (bitruss_msp.cu:537), which leaves the long tail

@@ -60,7 +60,11 @@ bt_status pack_range(const bt_graph *const *graphs, uint32_t first, uint32_t las
     out->u_max = U ? (uint32_t)(U - 1) : 0;
     out->support_max = 0;
     uint32_t max_n = 0;
-    for (uint32_t i = 0; i < k; i++) max_n = std::max(max_n, graphs[first + i]->n);
+    out->repeats = false;
+    for (uint32_t i = 0; i < k; i++) {
+        max_n = std::max(max_n, graphs[first + i]->n);
+        out->repeats |= graphs[first + i]->repeats;
+    }
     out->seg_max_n = max_n;
     try {
         out->segment.assign(out->n, 0);

@@ -75,6 +75,7 @@ struct CountArgs {
     uint32_t dense;      // counters in shared memory
     uint32_t batch;      // middle vertices at once: their suffixes' lengths are added in 32 bits
     uint32_t chunks;     // ceil(n / warps per CTA)
+    uint32_t least;      // middle slots from which a start vertex can close a butterfly
     uint32_t short_u, short_l;  // the other side's rows are short: for a start vertex in U, in L
     const uint32_t *off, *deg, *nbr, *is_u;
     const uint32_t *seg_base;  // per rank: first rank of its graph (NULL: one graph)
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
             const uint32_t mids = rl - lo;
             if (mids > kLightMids) {
                 big = r + 1;
-            } else if (mids > 1) {  // one middle vertex closes no butterfly
+            } else if (mids >= a.least) {
                 Mid m[kLightMids / 32];
                 uint32_t sum = 0;
 #pragma unroll
@@ -548,9 +549,14 @@ const void *count_kernel(bool per_edge, bool wide) {
 // CTAs of the counting kernel that hold counters in device memory
 int dev_count_ctas(bt_ctx *ctx) { return ctx->sm_count; }
 
-// Supports are summed in 64 bits when one could pass 2^32: a support is below
-// the product of its ends' degrees.
-static bool wide_sums(const DevGraph &g) { return (uint64_t)g.max_deg_u * g.max_deg_l > 0xffffffffull; }
+// Supports are summed in 64 bits where rows repeat a neighbour: with k parallel
+// edges r-s and k parallel edges s-w, each slot of r-s gets k (k^2 - 1) (2^32 from
+// k = 1,626 on).  Elsewhere each butterfly of an edge has an opposite edge of its
+// own, so no support and no slot's sum reaches m < 2^31.
+static bool wide_sums(const DevGraph &g) { return g.repeats; }
+
+// One middle slot alone closes a butterfly only if its row repeats an end.
+static uint32_t least_mids(const DevGraph &g) { return g.repeats ? 1 : 2; }
 
 uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide) {
     return (wide ? 16 : 8) * m + (span > kDense ? 8 * span * ctas : 0) + 1024;
@@ -596,6 +602,7 @@ bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count) {
     a.chunks = chunks;
     a.batch = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kBatch, 0xffffffffull / (g.max_deg + 1ull)));
     a.seg_base = g.seg_base;
+    a.least = least_mids(g);
     a.short_u = g.max_deg_l <= kShortRow;
     a.short_l = g.max_deg_u <= kShortRow;
     a.is_u = g.is_u;
@@ -655,6 +662,7 @@ bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *de
     a.dense = dense_of(n);
     a.chunks = (n + kCountWarps - 1) / kCountWarps;
     a.batch = (uint32_t)std::min<uint64_t>(kBatch, 0xffffffffull / n);  // degrees are below n
+    a.least = 2;  // no row repeats a neighbour
     a.off = off;
     a.deg = deg;
     a.nbr = nbr;

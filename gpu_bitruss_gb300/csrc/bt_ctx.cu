@@ -326,6 +326,7 @@ bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *hg) {
     g.n = n;
     g.m = m;
     g.u_num = hg->u_num;
+    g.repeats = hg->repeats;
     for (uint32_t x = 0; x < n; x++) {
         const uint32_t d = hg->degrees[x];
         uint32_t &side = x < g.u_num ? g.max_deg_u : g.max_deg_l;

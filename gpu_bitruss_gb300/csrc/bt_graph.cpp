@@ -18,6 +18,13 @@ namespace {
 
 constexpr uint32_t kMaxIds = 99999999u;  // MAX_IDS, src/util/config.h:6
 
+// A row's entries ascend strictly.
+bool ascending(const uint32_t *p, const uint32_t *end) {
+    for (; p < end && p + 1 < end; p++)
+        if (p[0] >= p[1]) return false;
+    return true;
+}
+
 // Build the CSR from an edge list in file order.  U and V ids are numbered by
 // first appearance (graph.cpp:99-105), V ids offset by u_num (:118-131), rows
 // sorted (:134-143), edge ids assigned to U slots in order (:178-194) and the
@@ -77,8 +84,13 @@ bt_status build_csr(const uint32_t *us, const uint32_t *vs, uint64_t m, bt_graph
     }
     uint32_t *nb = g->neighbors.data();
     const uint32_t *off = g->offsets.data();
-#pragma omp parallel for schedule(dynamic, 1024)
-    for (int64_t x = 0; x < (int64_t)n; x++) std::sort(nb + off[x], nb + off[x + 1]);
+    bool repeats = false;
+#pragma omp parallel for schedule(dynamic, 1024) reduction(|| : repeats)
+    for (int64_t x = 0; x < (int64_t)n; x++) {
+        std::sort(nb + off[x], nb + off[x + 1]);
+        if (!ascending(nb + off[x], nb + off[x + 1])) repeats = true;
+    }
+    g->repeats = repeats;
     // U rows occupy slots [0, m): slot s of a U row is edge s.
     for (uint32_t u = 0; u < u_num; u++) {
         for (uint32_t s = off[u]; s < off[u + 1]; s++) {
@@ -304,6 +316,8 @@ extern "C" bt_status bt_graph_load_bin(const char *path, bt_graph **out) {
         if (g->neighbors[s] >= n || g->edge_ids[s] >= m)
             return bt_fail(BT_ERR_FORMAT, std::string(path) + ": neighbour or edge id out of range");
     }
+    for (uint64_t x = 0; x < n && !g->repeats; x++)
+        g->repeats = !ascending(g->neighbors.data() + g->offsets[x], g->neighbors.data() + g->offsets[x + 1]);
     for (uint64_t e = 0; e < m; e++) {
         if (g->edges[2 * e] >= u_num || g->edges[2 * e + 1] < u_num || g->edges[2 * e + 1] >= n)
             return bt_fail(BT_ERR_FORMAT, std::string(path) + ": edge endpoints out of range");

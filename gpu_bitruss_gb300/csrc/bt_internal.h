@@ -58,6 +58,9 @@ struct bt_graph {
     std::vector<uint32_t> edge_ids;   // 2m
     std::vector<uint32_t> edge_support_raw;  // m, as stored in a .bin (int32 bits)
     std::vector<uint32_t> bitruss_raw;       // m, as stored in a .bin
+    // a row may hold a neighbour twice (duplicate lines are kept): some row does
+    // not ascend strictly
+    bool repeats = false;
     // batched arena only: graph index of every vertex (empty for one graph)
     // and the vertex count of the largest graph
     std::vector<uint32_t> segment;
@@ -79,6 +82,7 @@ struct DevGraph {
     uint64_t m = 0;
     uint32_t max_deg = 0;
     uint32_t max_deg_u = 0, max_deg_l = 0;  // largest degree of either side
+    bool repeats = false;       // a row may hold a neighbour twice
     uint32_t *off = nullptr;    // n+1 row starts
     uint32_t *deg0 = nullptr;   // n   degree
     uint32_t *nbr0 = nullptr;   // 2m  neighbour rank, ascending per row
@@ -164,11 +168,11 @@ void ctx_release_graph(bt_ctx *ctx);
 // most bytes the counting kernel's scratch takes (bt_count.cu)
 uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide);
 
-// Butterflies of one graph given by ranks, its rows in any order, on one CTA per
-// SM with counters in shared memory only; every buffer is the caller's and
-// nothing is allocated.  Degrees are below n, n < 2^31.  *next_chunk is zero on
-// entry; nothing is counted if *skip is not (bt_count.cu).  The set-up is made
-// once per device and context.
+// Butterflies of one graph given by ranks, its rows in any order and without a
+// neighbour twice, on one CTA per SM with counters in shared memory only; every
+// buffer is the caller's and nothing is allocated.  Degrees are below n, n < 2^31.
+// *next_chunk is zero on entry; nothing is counted if *skip is not (bt_count.cu).
+// The set-up is made once per device and context.
 bt_status bt_count_any_order_setup();
 bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *deg, const uint32_t *nbr,
                              unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st);

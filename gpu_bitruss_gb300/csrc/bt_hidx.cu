@@ -75,8 +75,10 @@ constexpr int kLightThreads = 256, kHeavyThreads = 256;
 // (1,024 and 16,384 were 1-5% slower on four graphs).
 constexpr float kLightPositions = 4096.0f;
 
-// N32: every value is below 2^32 - 1; values lie beside the slots and in the
-// tables.  Else 64-bit values, read through the edge ids in both places.
+// N32: every value is below 2^32 - 1 and no row repeats a neighbour; values lie
+// beside the slots and in the tables.  Else 64-bit values, read through the edge
+// ids in both places (the slots of parallel edges may share an edge id, and
+// set_value finds one slot per pair of ends).
 template <bool N32>
 using Val = typename std::conditional<N32, uint32_t, unsigned long long>::type;
 
@@ -631,6 +633,6 @@ bt_status dev_hidx(bt_ctx *ctx, uint32_t *rounds) {
     }
     // no value exceeds the largest support (BT_MSP_WIDE=1: as in the peel)
     const char *wide = getenv("BT_MSP_WIDE");
-    if (ctx->last_sup_max < 0xffffffffull && !(wide && *wide == '1')) return run_hidx<true>(ctx, from_peel, rounds);
+    if (ctx->last_sup_max < 0xffffffffull && !ctx->g.repeats && !(wide && *wide == '1')) return run_hidx<true>(ctx, from_peel, rounds);
     return run_hidx<false>(ctx, from_peel, rounds);
 }

@@ -63,3 +63,18 @@ def test_batch_with_and_without(engine, gpu_ctx, oracle_mod):
         want, total = oracle_mod.ebfc(oracle_mod.build_csr(u, v), 0)
         np.testing.assert_array_equal(sup, want)
         assert int(count) == total
+
+
+# Parallel edges may share an edge id and a table entry; an h-index value that
+# changes has to change wherever it is read.  64-bit values are read through the
+# edge ids, so both widths must end alike.
+@pytest.mark.parametrize("nu,nv,m,again,seed", [(60, 80, 1500, 20, 4), (500, 400, 8000, 400, 6), (20, 30, 150, 2, 20)])
+def test_hidx_values_of_parallel_edges(engine, gpu_ctx, nu, nv, m, again, seed, monkeypatch):
+    u, v = _repeated(nu, nv, m, again, seed)
+    gpu_ctx.upload(engine.Graph.from_edges(u.astype(np.uint32), v.astype(np.uint32)))
+    got = []
+    for wide in ("0", "1"):
+        monkeypatch.setenv("BT_MSP_WIDE", wide)
+        got.append(gpu_ctx.hidx())
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    assert got[0][1] == got[1][1]

@@ -78,6 +78,8 @@ struct CountArgs {
     uint32_t least;      // middle slots from which a start vertex can close a butterfly
     uint32_t short_u, short_l;  // the other side's rows are short: for a start vertex in U, in L
     const uint32_t *off, *deg, *nbr, *is_u;
+    const uint2 *rows;   // ANY_ORDER: off and deg side by side (then null)
+    uint32_t slots;      // ANY_ORDER: entries of nbr
     const uint32_t *seg_base;  // per rank: first rank of its graph (NULL: one graph)
     uint32_t *cnt;       // gridDim.x * span counters of ranks past the dense ones (zero on entry and exit)
     uint32_t *touched;   // gridDim.x * span
@@ -103,6 +105,18 @@ __device__ __forceinline__ void acc_add(void *acc, uint32_t slot, unsigned long 
     else atomicAdd(static_cast<uint32_t *>(acc) + slot, (uint32_t)v);
 }
 
+// r's first slot and its degree.  ANY_ORDER: the tables may be another call's by
+// now (bt_noalloc.cu); a row that does not end where the next one starts, as all
+// do there, is taken as empty.
+template <bool ANY_ORDER>
+__device__ __forceinline__ uint2 row_of(const CountArgs &a, uint32_t r) {
+    if (!ANY_ORDER) return make_uint2(__ldg(a.off + r), __ldg(a.deg + r));
+    const uint2 row = __ldg(a.rows + r);
+    const uint32_t next = r + 1 < a.n ? __ldg(&a.rows[r + 1].x) : a.slots;
+    const bool fits = next <= a.slots && row.x <= next && row.y == next - row.x && row.y < a.n;
+    return fits ? row : make_uint2(0, 0);
+}
+
 // 32 middle vertices of r, one per lane: where the suffix of ranks above r
 // starts in each one's row, and its length (0 past the end of r's row).
 // ANY_ORDER: rows are not sorted; the whole row of a middle vertex above r is
@@ -115,7 +129,9 @@ __device__ __forceinline__ Mid load_mid(const CountArgs &a, uint32_t rb, uint32_
     Mid m{0, 0};
     if (i < rl) {
         const uint32_t s = __ldg(a.nbr + rb + i);
-        const uint32_t sb = __ldg(a.off + s), sl = __ldg(a.deg + s);
+        if (ANY_ORDER && s >= a.n) return m;
+        const uint2 row = row_of<ANY_ORDER>(a, s);
+        const uint32_t sb = row.x, sl = row.y;
         const uint32_t j0 = ANY_ORDER ? (s > r ? 0 : sl) : upper_bound_u32(a.nbr + sb, sl, r);
         m.p0 = sb + j0;
         m.len = sl - j0;
@@ -321,7 +337,8 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
                                                          uint32_t r, uint32_t skip) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t base = a.seg_base ? a.seg_base[r] : 0u;
-    const uint32_t rb = a.off[r], rl = a.deg[r];
+    const uint2 row = row_of<ANY_ORDER>(a, r);
+    const uint32_t rb = row.x, rl = row.y;
     const uint32_t start = ANY_ORDER ? 0 : upper_bound_u32(a.nbr + rb, rl, r);
     uint32_t *cnt = a.cnt + (size_t)blockIdx.x * a.span;
     uint32_t *touched = a.touched + (size_t)blockIdx.x * a.span;
@@ -337,7 +354,7 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
         if (d < near) {
             atomicAdd(dense + d, 1u);
         } else if (ANY_ORDER) {
-            if (w > r && d - near < 0x80000000u) sm.touched = 1;  // ranks past these: another pass
+            if (w > r && w < a.n && d - near < 0x80000000u) sm.touched = 1;  // ranks past these: another pass
         } else if (a.span > a.dense && w - base < a.span) {
             const uint32_t old = atomicAdd(cnt + (w - base), 1u);
             local += old;
@@ -385,8 +402,10 @@ __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, Cou
         }
     } else {
         uint32_t nm = 0;
+        uint64_t seen = 0;
         for (uint32_t i0 = start; i0 < rl; i0 += a.batch) {
             nm = load_batch<ANY_ORDER>(a, sm, rb, rl, i0, r);
+            if (ANY_ORDER && (seen += sm.pre[nm]) > a.slots) break;  // no graph's: its rows share no slots
             visit_batch(a.nbr, sm, nm, [&](bool on, uint32_t w, uint32_t, uint32_t, bool) {
                 if (on) count_wedge(w);
             });
@@ -441,11 +460,10 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
     CountSmem &sm = *reinterpret_cast<CountSmem *>(smem_raw);
     uint32_t *dense = reinterpret_cast<uint32_t *>(smem_raw + sizeof(CountSmem));  // also the warps' hashes
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (ANY_ORDER && *a.layout_error) return;  // nothing to count here: see bt_count_any_order
     const uint32_t words = a.dense > kCountWarps * 2 * kSlots ? a.dense : kCountWarps * 2 * kSlots;
     uint4 *d4 = reinterpret_cast<uint4 *>(dense);
     for (uint32_t k = threadIdx.x; k < words / 4; k += kCountThreads) d4[k] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
+    if (__syncthreads_or(ANY_ORDER && *a.layout_error)) return;  // nothing to count here: see bt_count_any_order
     uint32_t *table = dense + warp * 2 * kSlots;
     unsigned long long local = 0;
     for (uint32_t c = blockIdx.x; c < a.chunks;) {
@@ -453,7 +471,8 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
         const uint32_t r = warp * a.chunks + c;
         uint32_t big = 0;
         if (r < a.n) {
-            const uint32_t rb = __ldg(a.off + r), rl = __ldg(a.deg + r);
+            const uint2 row = row_of<ANY_ORDER>(a, r);
+            const uint32_t rb = row.x, rl = row.y;
             // the suffix of r's own row after r, found 32 ways at a time
             uint32_t lo = 0, hi = ANY_ORDER ? 0 : rl;
             while (hi > lo) {
@@ -655,7 +674,7 @@ bt_status bt_count_any_order_setup() {
     return BT_OK;
 }
 
-bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *deg, const uint32_t *nbr,
+bt_status bt_count_any_order(uint32_t n, uint32_t slots, const uint2 *rows, const uint32_t *nbr,
                              unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st) {
     CountArgs a{};
     a.n = a.span = n;
@@ -663,9 +682,9 @@ bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *de
     a.chunks = (n + kCountWarps - 1) / kCountWarps;
     a.batch = (uint32_t)std::min<uint64_t>(kBatch, 0xffffffffull / n);  // degrees are below n
     a.least = 2;  // no row repeats a neighbour
-    a.off = off;
-    a.deg = deg;
+    a.rows = rows;
     a.nbr = nbr;
+    a.slots = slots;
     a.count = count;
     a.next_chunk = next_chunk;
     a.layout_error = skip;

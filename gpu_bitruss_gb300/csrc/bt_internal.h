@@ -170,11 +170,14 @@ uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide);
 
 // Butterflies of one graph given by ranks, its rows in any order and without a
 // neighbour twice, on one CTA per SM with counters in shared memory only; every
-// buffer is the caller's and nothing is allocated.  Degrees are below n, n < 2^31.
+// buffer is the caller's and nothing is allocated.  rows holds each rank's first
+// slot and degree (below n, n < 2^31), the rows one after the other; nbr has `slots`
+// entries.  Where the tables are not those of a graph the count
+// is wrong, but nothing outside them is read.
 // *next_chunk is zero on entry; nothing is counted if *skip is not (bt_count.cu).
 // The set-up is made once per device and context.
 bt_status bt_count_any_order_setup();
-bt_status bt_count_any_order(uint32_t n, const uint32_t *off, const uint32_t *deg, const uint32_t *nbr,
+bt_status bt_count_any_order(uint32_t n, uint32_t slots, const uint2 *rows, const uint32_t *nbr,
                              unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st);
 
 // algorithm entry points implemented in the .cu files

@@ -34,8 +34,12 @@
 //
 // All calls share the array: calls that overlap on the GPU (on different
 // streams or threads, without ordering between them) race on it and give
-// wrong counts.  The array keeps the last call's contents; each call clears
-// the parts that must start at zero (its counters and the work counter).
+// wrong counts, but touch nothing outside the array and the callers' buffers:
+// an index that comes from the array is compared with its range before it is
+// used, loops end whatever the array holds, and a block takes a branch that has
+// block barriers behind it on one answer for all its threads.  The array keeps
+// the last call's contents; each call clears the parts that must start at zero
+// (its counters and the work counter).
 //
 // The first call on a device looks up the array's device address with
 // cudaGetSymbolAddress (the host-side name of a __device__ array is only a
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(kThreadsNA) k_bfc_noalloc(uint32_t n, const ui
                                                             const uint32_t *only_if, unsigned long long *count) {
     __shared__ uint32_t s_r, s_nt;
     __shared__ unsigned long long s_red[kThreadsNA / 32];
-    if (only_if && !*only_if) return;
+    if (only_if && !__syncthreads_or(*only_if != 0)) return;
     uint32_t *cnt = scratch + (size_t)blockIdx.x * 2 * n;
     uint32_t *touched = cnt + n;
     for (uint32_t x = threadIdx.x; x < n; x += blockDim.x) cnt[x] = 0;  // left over from the last call
@@ -140,12 +144,18 @@ __global__ void __launch_bounds__(kThreadsNA) k_bfc_noalloc(uint32_t n, const ui
                 if (!higher(off, u, w)) continue;
                 const uint32_t old = atomicAdd(cnt + w, 1u);
                 local += old;
-                if (old == 0) touched[atomicAdd(&s_nt, 1u)] = w;
+                if (old == 0) {
+                    const uint32_t at = atomicAdd(&s_nt, 1u);
+                    if (at < n) touched[at] = w;
+                }
             }
         }
         __syncthreads();
-        const uint32_t nt = s_nt;
-        for (uint32_t k = threadIdx.x; k < nt; k += blockDim.x) cnt[touched[k]] = 0;
+        const uint32_t nt = min(s_nt, n);
+        for (uint32_t k = threadIdx.x; k < nt; k += blockDim.x) {
+            const uint32_t w = touched[k];
+            if (w < n) cnt[w] = 0;
+        }
         __syncthreads();
     }
     for (int o = 16; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
@@ -171,7 +181,9 @@ struct Ranks {
     uint32_t *bins;   // per degree: its vertices, then the rank of the first (zero on entry)
     uint32_t *taken;  // per degree: ranks given out (zero on entry)
     uint32_t *slots;  // per degree: first row slot
-    uint32_t *rank, *off, *deg, *nbr;
+    uint32_t *rank;
+    uint2 *rows;      // per rank: first row slot, degree (2n words)
+    uint32_t *nbr;
 };
 
 // Vertices per degree and the largest degree.  The later kernels' indexes rest
@@ -197,10 +209,13 @@ __global__ void k_na_degrees(uint32_t n, uint64_t m, const uint32_t *off, Ranks 
 
 // Per degree, the first rank and the first row slot of its vertices, largest
 // degree first; one block.
-__global__ void __launch_bounds__(1024) k_na_scan(Ranks t, const Words *w) {
+__global__ void __launch_bounds__(1024) k_na_scan(uint32_t n, Ranks t, const Words *w) {
     __shared__ unsigned long long s_warp[32];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, top = w->largest;
-    if (w->irregular) return;
+    __shared__ uint32_t s_top;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_top = min(w->largest, n - 1);
+    if (__syncthreads_or(w->irregular != 0)) return;
+    const uint32_t top = s_top;
     unsigned long long run = 0;
     for (uint32_t i0 = 0; i0 <= top; i0 += 1024) {
         const uint32_t i = i0 + threadIdx.x, d = top - i;  // degrees downwards
@@ -237,6 +252,7 @@ __global__ void k_na_rank(uint32_t n, const uint32_t *off, Ranks t, const Words 
     if (w->irregular) return;
     for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
         const uint32_t d = off[x + 1] - off[x];
+        if (d >= n) continue;
         // the lanes of one degree take their ranks together
         const uint32_t on = __activemask(), same = __match_any_sync(on, d);
         const uint32_t lane = threadIdx.x & 31, lead = __ffs(same) - 1;
@@ -244,9 +260,9 @@ __global__ void k_na_rank(uint32_t n, const uint32_t *off, Ranks t, const Words 
         if (lane == lead) k = atomicAdd(t.taken + d, (uint32_t)__popc(same));
         k = __shfl_sync(same, k, lead) + __popc(same & ((1u << lane) - 1));
         const uint32_t r = t.bins[d] + k;
+        if (r >= n) continue;
         t.rank[x] = r;
-        t.off[r] = t.slots[d] + k * d;
-        t.deg[r] = d;
+        t.rows[r] = make_uint2(t.slots[d] + k * d, d);
     }
 }
 
@@ -261,7 +277,9 @@ __global__ void k_na_rows(uint32_t n, const uint32_t *off, const uint32_t *nbr, 
         const uint32_t y = nbr[p], before = p ? nbr[p - 1] : 0;
         const uint32_t x = bt::row_of_slot(off, n, (uint32_t)p), j = (uint32_t)p - off[x];
         if (y >= n || (j && before >= y)) bad = true;
-        t.nbr[t.off[t.rank[x]] + j] = y < n ? t.rank[y] : 0;
+        const uint32_t r = t.rank[x];
+        const uint64_t dst = r < n ? (uint64_t)t.rows[r].x + j : slots;
+        if (dst < slots) t.nbr[dst] = y < n ? t.rank[y] : 0;
     }
     if (bad) w->irregular = 1;
 }
@@ -319,17 +337,17 @@ extern "C" bt_status bt_bfc_noalloc(int device, const uint32_t *d_offsets, const
     const bool by_rank = m >= kRankEdges && 6ull * n + 2 * m <= kScratchWords;
     if (by_rank) {
         uint32_t *p = scratch;
-        const Ranks t{p, p + n, p + 2ull * n, p + 3ull * n, p + 4ull * n, p + 5ull * n, p + 6ull * n};
+        const Ranks t{p, p + n, p + 2ull * n, p + 3ull * n, reinterpret_cast<uint2 *>(p + 4ull * n), p + 6ull * n};
         BT_CUDA(cudaMemsetAsync(t.bins, 0, 8ull * n, st));  // and taken
         const unsigned most = (unsigned)sms * 8, per_vertex = std::min(most, (n + 255) / 256);
         const unsigned per_slot = (unsigned)std::min<uint64_t>(most, (2 * m + 255) / 256);
         k_na_degrees<<<per_vertex, 256, 0, st>>>(n, m, d_offsets, t, words);
-        k_na_scan<<<1, 1024, 0, st>>>(t, words);
+        k_na_scan<<<1, 1024, 0, st>>>(n, t, words);
         k_na_rank<<<per_vertex, 256, 0, st>>>(n, d_offsets, t, words);
         k_na_rows<<<per_slot, 256, 0, st>>>(n, d_offsets, d_neighbors, 2 * m, t, words);
         bt_note_launches(4);
         BT_CUDA(cudaGetLastError());
-        BT_TRY(bt_count_any_order(n, t.off, t.deg, t.nbr, d_count, &words->next_chunk, &words->irregular, sms, st));
+        BT_TRY(bt_count_any_order(n, (uint32_t)(2 * m), t.rows, t.nbr, d_count, &words->next_chunk, &words->irregular, sms, st));
     }
     uint64_t ctas = (uint64_t)sms * 2;
     const uint64_t fit = kScratchWords / (2ull * n);

@@ -50,7 +50,8 @@ namespace {
 constexpr int kCountThreads = 1024;
 constexpr uint32_t kCountWarps = kCountThreads / 32;
 constexpr uint32_t kDense = 52224;         // counters in shared memory (204 KiB)
-constexpr uint32_t kBatch = kCountThreads; // middle vertices a CTA lays end to end at once
+constexpr uint32_t kBatch = kCountBatch;   // middle vertices a CTA lays end to end at once
+static_assert(kCountBatch == kCountThreads && kCountStride == kCountThreads * 4, "one per thread; four positions each");
 // Longest row a single warp may have to walk by itself.  On the hub-skewed
 // graph (rows of at most 60) warps on their own take 1.1 ms, batches of the
 // CTA 1.7; on the Chung-Lu graph (rows of up to 10k) 5.7 and 2.6.
@@ -291,7 +292,7 @@ template <class F>
 __device__ __forceinline__ void visit_batch(const uint32_t *nbr, const CountSmem &sm, uint32_t nm, F f) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t total = sm.pre[nm];
-    for (uint32_t fb = warp * 128; fb < total; fb += kCountThreads * 4) {
+    for (uint32_t fb = warp * 128; fb < total; fb += kCountStride) {
         // the middle vertex of position fb
         uint32_t k0 = 0, hi = nm;
         while (hi - k0 > 1) {
@@ -619,7 +620,7 @@ bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count) {
     a.span = (uint32_t)span;
     a.dense = dense;
     a.chunks = chunks;
-    a.batch = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(kBatch, 0xffffffffull / (g.max_deg + 1ull)));
+    a.batch = bt_count_batch(g.max_deg);
     a.seg_base = g.seg_base;
     a.least = least_mids(g);
     a.short_u = g.max_deg_l <= kShortRow;
@@ -680,7 +681,7 @@ bt_status bt_count_any_order(uint32_t n, uint32_t slots, const uint2 *rows, cons
     a.n = a.span = n;
     a.dense = dense_of(n);
     a.chunks = (n + kCountWarps - 1) / kCountWarps;
-    a.batch = (uint32_t)std::min<uint64_t>(kBatch, 0xffffffffull / n);  // degrees are below n
+    a.batch = bt_count_batch(n - 1);  // degrees are below n
     a.least = 2;  // no row repeats a neighbour
     a.rows = rows;
     a.nbr = nbr;

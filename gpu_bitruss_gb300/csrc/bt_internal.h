@@ -165,6 +165,18 @@ bt_status ctx_alloc_t(bt_ctx *ctx, T **p, uint64_t count) {
 bt_status ctx_scratch(bt_ctx *ctx, uint64_t bytes, void **p);
 void ctx_release_graph(bt_ctx *ctx);
 
+// Middle vertices whose wedges the counting kernel lays end to end at once, at
+// most, and the positions its warps go on by.
+constexpr uint32_t kCountBatch = 1024, kCountStride = 4096;
+
+// As many of them as can be laid end to end where no row is longer: positions are
+// 32-bit numbers, also the one a warp reaches past the last.  (With repeated
+// lines the rows of a batch may all be the longest.)
+inline uint32_t bt_count_batch(uint32_t longest_row) {
+    const uint64_t fit = (0xffffffffull - kCountStride) / (longest_row + 1ull);
+    return fit < 1 ? 1 : fit < kCountBatch ? (uint32_t)fit : kCountBatch;
+}
+
 // most bytes the counting kernel's scratch takes (bt_count.cu)
 uint64_t bt_count_bytes(uint64_t m, uint64_t span, uint64_t ctas, bool wide);
 

@@ -1,0 +1,16 @@
+"""Host-side parts of the engine's headers, compiled and run without a GPU."""
+
+import os
+import subprocess
+
+from conftest import ROOT
+
+
+def test_host_units(tmp_path):
+    src = os.path.join(ROOT, "tests", "cpp", "host_units.cpp")
+    exe = str(tmp_path / "host_units")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    r = subprocess.run(["g++", "-O1", "-std=c++17", "-I", cuda, src, "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout

@@ -79,12 +79,13 @@ uint64_t tab_buckets_of(const bt_graph *g) {
 
 // Device bytes a job on an arena of these sizes allocates at its peak (every
 // array of dev_build_graph, dev_ebfc and dev_msp; CUB temporaries bounded
-// above).  count_ctas: resident CTAs of the counting kernel.
+// above).  count_ctas: resident CTAs of the counting kernel; repeats: some graph's
+// rows may repeat a neighbour, its supports are then summed in 64 bits.
 uint64_t bt_job_footprint(uint64_t n, uint64_t m, uint64_t tab_buckets, uint64_t span,
-                          uint64_t count_ctas, uint64_t graphs, bool peel) {
+                          uint64_t count_ctas, uint64_t graphs, bool repeats, bool peel) {
     const uint64_t resident = 36 * m + 16 * n + (1u << 16);
     const uint64_t upload = 32 * m + 52 * n + (16 * m + 24 * n + (4u << 20));
-    const uint64_t count = bt_count_bytes(m, span, count_ctas, true) + (1u << 16);
+    const uint64_t count = bt_count_bytes(m, span, count_ctas, repeats) + (1u << 16);
     const uint64_t msp = peel ? 52 * m + 16 * n + 32 * tab_buckets + 2048 * graphs + (1u << 16) : 0;
     return resident + std::max(upload, count + msp);
 }
@@ -96,14 +97,16 @@ extern "C" bt_status bt_job_bytes(bt_ctx *ctx, const bt_graph *const *graphs, ui
     if (!ctx || !bytes || (count && !graphs)) return bt_fail(BT_ERR_INVALID, "null argument");
     if (op < BT_OP_BFC || op > BT_OP_MSP_EXACT) return bt_fail(BT_ERR_INVALID, "unknown op");
     uint64_t n = 0, m = 0, tab = 0, span = 0;
+    bool repeats = false;
     for (uint32_t i = 0; i < count; i++) {
         if (!graphs[i]) return bt_fail(BT_ERR_INVALID, "null graph");
         n += graphs[i]->n;
         m += graphs[i]->m;
         tab += tab_buckets_of(graphs[i]);
         span = std::max<uint64_t>(span, graphs[i]->n);
+        repeats |= graphs[i]->repeats;
     }
-    *bytes = bt_job_footprint(n, m, tab, span, (uint64_t)dev_count_ctas(ctx), count, kind_of(op) != 0);
+    *bytes = bt_job_footprint(n, m, tab, span, (uint64_t)dev_count_ctas(ctx), count, repeats, kind_of(op) != 0);
     return BT_OK;
 }
 
@@ -125,13 +128,15 @@ struct bt_server {
 
     uint64_t footprint(const std::vector<ReqPtr> &job) const {
         uint64_t n = 0, m = 0, tab = 0, span = 0;
+        bool repeats = false;
         for (const auto &r : job) {
             n += r->g->n;
             m += r->g->m;
             tab += r->tab_buckets;
             span = std::max<uint64_t>(span, r->g->n);
+            repeats |= r->g->repeats;
         }
-        return bt_job_footprint(n, m, tab, span, count_ctas, job.size(), kind_of(job[0]->op) != 0);
+        return bt_job_footprint(n, m, tab, span, count_ctas, job.size(), repeats, kind_of(job[0]->op) != 0);
     }
 
     // pick a job (lock held); empty if nothing can start now

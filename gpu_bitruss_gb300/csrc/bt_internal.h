@@ -147,6 +147,26 @@ struct bt_ctx {
     uint32_t peel_ctas = 0;             // CTAs of the peeling kernel (0 = one per SM)
 };
 
+// Counters of one thread of the peel (a warp's positions are its first lane's).
+// They pass 2^32: the 10M-edge hub graph walks 1.4e12 positions, 4.5e9 a warp on an
+// eighth of the SMs.  In 64 bits they cost the kernel 16 bytes of spills, so
+// each keeps 31 and a task's end carries what is above to the totals.  A task
+// adds less than 2^31 to each.
+struct PeelWork {
+    uint32_t probes = 0, hits = 0, decs = 0;
+    __host__ __device__ bool full() const { return (probes | hits | decs) >> 31; }
+    // totals: the sums in 64 bits, which add(address, value) adds to
+    template <class S, class Add>
+    __host__ __device__ void carry(S &totals, Add add) {
+        add(&totals.w_probes, probes & 0x80000000u);
+        add(&totals.w_hits, hits & 0x80000000u);
+        add(&totals.w_decs, decs & 0x80000000u);
+        probes &= 0x7fffffffu;
+        hits &= 0x7fffffffu;
+        decs &= 0x7fffffffu;
+    }
+};
+
 // Default msp task schedule (bt_ctx_set_msp_schedule with 0 picks these):
 // probe positions per task, frontier chunks per CTA, whole-plan limit.
 constexpr uint32_t kMspMinGrain = 64;

@@ -182,11 +182,6 @@ struct Team {
     __device__ __forceinline__ uint32_t threads() const { return size * kThreads; }
 };
 
-// Counters of one thread.
-struct Work {
-    uint32_t probes = 0, hits = 0, decs = 0;
-};
-
 // Optional per-sub-round trace (BT_MSP_TRACE=<path>): what bounds a sub-round.
 struct TraceRow {
     unsigned long long t_ns;        // sub-round duration seen by CTA 0 (plan to barrier exit)
@@ -530,7 +525,7 @@ constexpr uint32_t kNbMask = 0x3fffffffu;
 // one by one; no block barriers.
 template <bool N32>
 __device__ __forceinline__ void run_tasks(const MspArgs &a, Smem &sm, uint32_t cnt, uint32_t tasks, uint32_t first,
-                                          uint32_t step, const Round<N32> &rd, Work &wk, SupWord<N32> &low) {
+                                          uint32_t step, const Round<N32> &rd, PeelWork &wk, SupWord<N32> &low) {
     const uint32_t lane = threadIdx.x & 31, r = rd.r;
     uint32_t *dec = sm.dec + (threadIdx.x & ~31u);
     for (uint32_t task = first + step * (threadIdx.x >> 5); task < tasks;) {
@@ -624,6 +619,7 @@ __device__ __forceinline__ void run_tasks(const MspArgs &a, Smem &sm, uint32_t c
             old[2] = dec_issue<N32>(a, e_pm, n_pm);
         }
         dec_settle<N32>(a, rd, pe, n_pm, old, low);
+        if (wk.full()) wk.carry(*a.sh, [](unsigned long long *t, uint32_t v) { atomicAdd(t, (unsigned long long)v); });
         __syncwarp();
         task = first + step * __shfl_sync(0xffffffffu, j, 0);
     }
@@ -633,7 +629,7 @@ __device__ __forceinline__ void run_tasks(const MspArgs &a, Smem &sm, uint32_t c
 // has planned it already when it is short).
 template <bool N32>
 __device__ __forceinline__ void peel(const MspArgs &a, const Team &t, Smem &sm, const uint32_t *curr, uint32_t len, uint32_t *ctr,
-                                     const Round<N32> &rd, Work &wk, SupWord<N32> &low) {
+                                     const Round<N32> &rd, PeelWork &wk, SupWord<N32> &low) {
     const uint32_t rank = t.rank, size = t.size;
     // a frontier that every CTA plans whole, its tasks dealt to all CTAs, or
     // chunks of it that a CTA plans and runs alone: its first is its own
@@ -752,7 +748,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
     t.bar = &team->bar;
     const uint32_t gtid = t.thread(), gsz = t.threads();
     const bool clerk = t.rank == 0 && is_clerk();
-    Work wk;
+    PeelWork wk;
     uint32_t epoch = 0;               // barrier arrivals so far (the same in every CTA of the team)
     // of the team's clerk
     const unsigned long long t_start = bt::global_ns(), c_start = clock64();
@@ -925,7 +921,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
             prof_mark(sm, PF_PROBE);
             fold_low<N32>(sm, low);
             if (a.trace && r < a.trace_cap) {
-                const unsigned long long walked = warp_sum(wk.probes - probes0);
+                // (less than 2^31 a warp; bit 31 may have been carried meanwhile)
+                const unsigned long long walked = warp_sum((wk.probes - probes0) & 0x7fffffffu);
                 if ((threadIdx.x & 31) == 0) {
                     atomicMax(&a.trace[r].max_task_ns, bt::global_ns() - task_t0);
                     atomicAdd(&a.trace[r].walked, walked);

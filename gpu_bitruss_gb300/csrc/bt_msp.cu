@@ -862,7 +862,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
                     fold_low<N32>(sm, low);
                     squeeze = (double)live <= (double)a.cfrac * (double)live_at_compress &&
                               (double)live_at_compress >= (double)a.cfloor * (double)t.job.m;
-                    if (!barrier(a, t, sm, epoch, k3, sm.now.scan_len[k3], r & 1, true)) return;
+                    // (a compaction changes the rows that a plan is made from: it comes after it)
+                    if (!barrier(a, t, sm, epoch, k3, sm.now.scan_len[k3], r & 1, !squeeze)) return;
                     curr_len = sm.now.scan_len[k3];
                     if (compact) {
                         uint32_t *t = near0; near0 = near1; near1 = t;

@@ -93,6 +93,11 @@ bt_status ctx_alloc(bt_ctx *ctx, void **p, uint64_t bytes) {
         return bt_fail(BT_ERR_DEVICE_MEMORY, "device budget of " + std::to_string(ctx->budget) +
                                                  " bytes exceeded (need " +
                                                  std::to_string(ctx->used + bytes) + ")");
+    try {
+        if (ctx->allocs.size() == ctx->allocs.capacity()) ctx->allocs.reserve(2 * ctx->allocs.size() + 32);
+    } catch (const std::bad_alloc &) {
+        return bt_fail(BT_ERR_HOST_MEMORY, "host allocation failed");
+    }
     cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
     if (e != cudaSuccess) {
         *p = nullptr;

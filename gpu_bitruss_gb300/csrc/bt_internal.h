@@ -183,6 +183,30 @@ bt_status ctx_alloc_t(bt_ctx *ctx, T **p, uint64_t count) {
     return ctx_alloc(ctx, reinterpret_cast<void **>(p), count * sizeof(T));
 }
 bt_status ctx_scratch(bt_ctx *ctx, uint64_t bytes, void **p);
+
+// Device buffers of one call, given back when it ends, also by an exception.
+class CtxBuffers {
+public:
+    explicit CtxBuffers(bt_ctx *ctx) : ctx_(ctx) {}
+    ~CtxBuffers() {
+        for (void *p : held_) ctx_free(ctx_, p);
+    }
+    CtxBuffers(const CtxBuffers &) = delete;
+    CtxBuffers &operator=(const CtxBuffers &) = delete;
+    template <class T>
+    bt_status alloc(T **p, uint64_t bytes) {
+        held_.push_back(nullptr);  // may throw: before there is anything to lose
+        void *q = nullptr;
+        const bt_status s = ctx_alloc(ctx_, &q, bytes);
+        held_.back() = q;
+        *p = static_cast<T *>(q);
+        return s;
+    }
+
+private:
+    bt_ctx *ctx_;
+    std::vector<void *> held_;
+};
 void ctx_release_graph(bt_ctx *ctx);
 
 // Middle vertices whose wedges the counting kernel lays end to end at once, at

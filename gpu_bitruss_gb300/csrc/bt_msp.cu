@@ -1157,16 +1157,7 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     cudaEvent_t e0 = ctx->ev[2], e1 = ctx->ev[3];
     cudaEventRecord(e0, st);
 
-    std::vector<void *> owned;
-    auto alloc = [&](void **p, uint64_t bytes) -> bt_status {
-        bt_status r = ctx_alloc(ctx, p, bytes);
-        if (r == BT_OK) owned.push_back(*p);
-        return r;
-    };
-    auto release = [&]() {
-        for (void *p : owned) ctx_free(ctx, p);
-        owned.clear();
-    };
+    CtxBuffers buffers(ctx);
     // the graphs to peel, largest first, and how many CTAs peel each
     std::vector<Job> jobs;
     std::vector<uint2> by_edge;
@@ -1179,12 +1170,7 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     MspArgs a{};
     uint2 *d_by_edge = nullptr;
     const uint64_t mm = m ? m : 1, nn = n ? n : 1;
-    bt_status rc = BT_OK;
-#define A(p, bytes)                                       \
-    do {                                                  \
-        rc = alloc((void **)&(p), (bytes));               \
-        if (rc != BT_OK) { release(); return rc; }        \
-    } while (0)
+#define A(p, bytes) BT_TRY(buffers.alloc(&(p), (bytes)))
     A(a.sh, sizeof(MspShared));
     A(a.states, sizeof(MspState) * (njobs ? njobs : 1));
     A(a.jobs, sizeof(Job) * (njobs ? njobs : 1));
@@ -1213,18 +1199,13 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         A(a.trace, sizeof(TraceRow) * a.trace_cap);
     }
     a.result = ctx->result;
-#define C(x)                                                                  \
-    do {                                                                      \
-        cudaError_t _e = (x);                                                 \
-        if (_e != cudaSuccess) { release(); return bt_cuda_fail(_e, #x, __FILE__, __LINE__); } \
-    } while (0)
     // cooperative persistent launch: its CTAs, in teams
     const size_t smem = sizeof(Smem);
     const void *kfn = a.sup32 ? (const void *)k_msp<true> : (const void *)k_msp<false>;
-    C(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    C(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kThreads, smem));
-    if (per_sm < 1) { release(); return bt_fail(BT_ERR_CUDA, "msp kernel does not fit on an SM"); }
+    BT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kThreads, smem));
+    if (per_sm < 1) return bt_fail(BT_ERR_CUDA, "msp kernel does not fit on an SM");
     const uint32_t capacity = (uint32_t)(ctx->sm_count * per_sm);
     const uint32_t ctas = ctx->peel_ctas && ctx->peel_ctas < capacity ? ctx->peel_ctas : capacity;
     const std::vector<uint32_t> sizes = plan_teams(jobs, ctas);
@@ -1241,18 +1222,18 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     A(a.teams, sizeof(TeamState) * teams.size());
     A(a.team_of, 4 * team_of.size());
 #undef A
-    C(cudaMemsetAsync(a.sh, 0, sizeof(MspShared), st));
+    BT_CUDA(cudaMemsetAsync(a.sh, 0, sizeof(MspShared), st));
     // (these are copied before the calls return: pageable memory)
-    C(cudaMemcpyAsync(a.teams, teams.data(), sizeof(TeamState) * teams.size(), cudaMemcpyHostToDevice, st));
-    C(cudaMemcpyAsync((void *)a.team_of, team_of.data(), 4 * team_of.size(), cudaMemcpyHostToDevice, st));
-    C(cudaMemsetAsync(a.states, 0, sizeof(MspState) * (njobs ? njobs : 1), st));
+    BT_CUDA(cudaMemcpyAsync(a.teams, teams.data(), sizeof(TeamState) * teams.size(), cudaMemcpyHostToDevice, st));
+    BT_CUDA(cudaMemcpyAsync((void *)a.team_of, team_of.data(), 4 * team_of.size(), cudaMemcpyHostToDevice, st));
+    BT_CUDA(cudaMemsetAsync(a.states, 0, sizeof(MspState) * (njobs ? njobs : 1), st));
     if (njobs) {
-        C(cudaMemcpyAsync((void *)a.jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st));
-        C(cudaMemcpyAsync(d_by_edge, by_edge.data(), sizeof(uint2) * njobs, cudaMemcpyHostToDevice, st));
+        BT_CUDA(cudaMemcpyAsync((void *)a.jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st));
+        BT_CUDA(cudaMemcpyAsync(d_by_edge, by_edge.data(), sizeof(uint2) * njobs, cudaMemcpyHostToDevice, st));
     }
-    if (a.trace) C(cudaMemsetAsync(a.trace, 0, sizeof(TraceRow) * a.trace_cap, st));
-    C(cudaMemcpyAsync(a.nbr, g.nbr0, 8 * m, cudaMemcpyDeviceToDevice, st));
-    C(cudaMemcpyAsync(a.eid, g.eid0, 8 * m, cudaMemcpyDeviceToDevice, st));
+    if (a.trace) BT_CUDA(cudaMemsetAsync(a.trace, 0, sizeof(TraceRow) * a.trace_cap, st));
+    BT_CUDA(cudaMemcpyAsync(a.nbr, g.nbr0, 8 * m, cudaMemcpyDeviceToDevice, st));
+    BT_CUDA(cudaMemcpyAsync(a.eid, g.eid0, 8 * m, cudaMemcpyDeviceToDevice, st));
     a.njobs = njobs;
     a.n = g.n;
     a.m = m;
@@ -1286,12 +1267,10 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         k_msp_init<<<(unsigned)std::min<uint64_t>(blocks, cap), blk, 0, st>>>(
             a, (const unsigned long long *)ctx->sup, g.off, g.deg0, d_by_edge);
         bt_note_launches(1);
-        C(cudaGetLastError());
+        BT_CUDA(cudaGetLastError());
     }
-    if (ctx->device < 0 || ctx->device >= kMaxPoolDevices) {
-        release();
+    if (ctx->device < 0 || ctx->device >= kMaxPoolDevices)
         return bt_fail(BT_ERR_INVALID, "device index out of range");
-    }
     // SM slots (see CtaSlots): concurrent peels of this process fit side by side
     CtaSlots slots;
     NvtxRange range("k_msp");
@@ -1303,7 +1282,6 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         if (le == cudaSuccess) le = cudaGetLastError();
         if (le != cudaSuccess) {
             slots.release();
-            release();
             return bt_cuda_fail(le, "cudaLaunchCooperativeKernel(k_msp)", __FILE__, __LINE__);
         }
         cudaEventRecord(ctx->ev[5], st);
@@ -1315,30 +1293,25 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
         cudaError_t ce = cudaMemcpyAsync(&h, a.sh, sizeof(MspShared), cudaMemcpyDeviceToHost, st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
         slots.release();
-        if (ce != cudaSuccess) {
-            release();
-            return bt_cuda_fail(ce, "msp state readback", __FILE__, __LINE__);
-        }
+        if (ce != cudaSuccess) return bt_cuda_fail(ce, "msp state readback", __FILE__, __LINE__);
     }
     if (a.trace) {
         // rows 2 .. subrounds+1 are sub-rounds; written as raw TraceRow records
         const uint64_t rows = std::min<uint64_t>(h.subrounds + 2, a.trace_cap);
         std::vector<TraceRow> tr(rows);
-        C(cudaMemcpyAsync(tr.data(), a.trace, sizeof(TraceRow) * rows, cudaMemcpyDeviceToHost, st));
-        C(cudaStreamSynchronize(st));
+        BT_CUDA(cudaMemcpyAsync(tr.data(), a.trace, sizeof(TraceRow) * rows, cudaMemcpyDeviceToHost, st));
+        BT_CUDA(cudaStreamSynchronize(st));
         if (FILE *f = fopen(trace_path, "wb")) {
             fwrite(tr.data(), sizeof(TraceRow), rows, f);
             fclose(f);
         }
     }
-#undef C
     float ms = -1;
     cudaEventElapsedTime(&ms, e0, e1);
     ctx->phase_ms[PH_MSP] = ms;
     ms = -1;
     if (m) cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]);
     ctx->phase_ms[PH_PEEL] = ms;
-    release();
     if (h.error == bt::ERR_TIMEOUT)
         return bt_fail(BT_ERR_TIMEOUT, "msp: a grid barrier wait exceeded its time limit");
     if (h.overflow) return bt_fail(BT_ERR_OVERFLOW, "msp: a bitruss number exceeds uint32");

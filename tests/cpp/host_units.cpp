@@ -1,8 +1,9 @@
 // Host-side parts of the engine's headers, checked without a GPU: the largest
 // batch of middle vertices whose wedge positions are 32-bit numbers; the peel's
-// counters past 2^32.
+// counters past 2^32; the device buffers of a call that ends by an exception.
 #include <cstdint>
 #include <cstdio>
+#include <new>
 
 #include "../../gpu_bitruss_gb300/csrc/bt_internal.h"
 
@@ -46,4 +47,51 @@ static int peel_counters() {
     return 0;
 }
 
-int main() { return count_batch() || peel_counters(); }
+// stand-ins for the context's allocator: what is held, and one failing call
+static std::vector<void *> g_held;
+static int g_fail_at = -1, g_calls = 0;
+bt_status ctx_alloc(bt_ctx *, void **p, uint64_t) {
+    *p = nullptr;
+    if (g_calls++ == g_fail_at) return BT_ERR_DEVICE_MEMORY;
+    *p = new char;
+    g_held.push_back(*p);
+    return BT_OK;
+}
+void ctx_free(bt_ctx *, void *p) {
+    if (!p) return;
+    for (size_t i = 0; i < g_held.size(); i++)
+        if (g_held[i] == p) {
+            g_held.erase(g_held.begin() + (long)i);
+            delete static_cast<char *>(p);
+            return;
+        }
+    std::printf("freed twice\n");
+}
+static bt_status use_buffers(bool raise) {
+    CtxBuffers b(nullptr);
+    uint32_t *x = nullptr;
+    uint2 *y = nullptr;
+    BT_TRY(b.alloc(&x, 4));
+    BT_TRY(b.alloc(&y, 8));
+    if (!x || !y || g_held.size() != 2) return BT_ERR_STATE;
+    if (raise) throw std::bad_alloc();
+    return BT_OK;
+}
+static int call_buffers() {
+    CHECK(use_buffers(false) == BT_OK && g_held.empty());
+    bool caught = false;
+    try {
+        use_buffers(true);
+    } catch (const std::bad_alloc &) {
+        caught = true;
+    }
+    CHECK(caught && g_held.empty());
+    for (int k = 0; k < 2; k++) {
+        g_calls = 0;
+        g_fail_at = k;
+        CHECK(use_buffers(true) == BT_ERR_DEVICE_MEMORY && g_held.empty());
+    }
+    return 0;
+}
+
+int main() { return count_batch() || peel_counters() || call_buffers(); }

@@ -309,7 +309,7 @@ extern "C" bt_status bt_ctx_get_msp_schedule(const bt_ctx *ctx, uint32_t *out) {
 extern "C" bt_status bt_msp_autotune(bt_ctx *ctx, uint32_t *out, double *best_ms) {
     BT_TRY(enter_ctx(ctx));
     if (!ctx->has_graph) return bt_fail(BT_ERR_STATE, "no graph uploaded to this context");
-    static const uint32_t grains[] = {32, 64, 128, 256, 512};
+    static const uint32_t grains[] = {1024, 2048, 4096, 8192, 16384};
     static const uint32_t tasks[] = {1, 2, 4, 8};
     static const uint32_t plans[] = {64, 256, 512};
     uint32_t cur[3];

@@ -141,7 +141,7 @@ struct bt_ctx {
     cudaEvent_t ev[8] = {};
     uint64_t *host_words = nullptr;  // 4 page-locked words: a count's results come back without a staging copy
 
-    // msp task schedule (0 = built-in value): positions per task, chunks per CTA, whole-plan limit
+    // msp task schedule (0 = built-in value): positions per 32 tasks, chunks per CTA, whole-plan limit
     uint32_t msp_schedule[3] = {0, 0, 0};
     uint64_t arena_edges = 1ull << 28;  // batched calls: edges per arena, at most
     uint32_t peel_ctas = 0;             // CTAs of the peeling kernel (0 = one per SM)
@@ -168,8 +168,8 @@ struct PeelWork {
 };
 
 // Default msp task schedule (bt_ctx_set_msp_schedule with 0 picks these):
-// probe positions per task, frontier chunks per CTA, whole-plan limit.
-constexpr uint32_t kMspMinGrain = 64;
+// probe positions per 32 tasks, frontier chunks per CTA, whole-plan limit.
+constexpr uint32_t kMspMinGrain = 2048;
 constexpr uint32_t kMspTasksPerCta = 2;
 constexpr uint32_t kMspLocalPlan = 512;
 

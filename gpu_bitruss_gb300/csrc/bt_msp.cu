@@ -1238,7 +1238,7 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     a.n = g.n;
     a.m = m;
     a.exact = exact ? 1u : 0u;
-    a.inv_task = 1.0f / (float)(ctx->msp_schedule[0] ? ctx->msp_schedule[0] : kMspMinGrain);
+    a.inv_task = 32.0f / (float)(ctx->msp_schedule[0] ? ctx->msp_schedule[0] : kMspMinGrain);
     a.chunks_per_cta = ctx->msp_schedule[1] ? ctx->msp_schedule[1] : kMspTasksPerCta;
     a.local_plan = std::min(ctx->msp_schedule[2] ? ctx->msp_schedule[2] : kMspLocalPlan, kEdges);
     a.wait_ns = wait_limit_ns();

@@ -163,11 +163,11 @@ bt_status bt_ctx_stats(const bt_ctx *ctx, uint64_t *out, int n);
 
 /* ---- peeling schedule and its autotuner ------------------------------- */
 
-/* The msp task schedule.  min_grain: probe positions a peel task (one warp)
- * should hold; tasks_per_cta: chunks per CTA that a frontier too large to be
- * planned whole is cut into; local_plan: frontiers of at most this many edges
- * (<= 512) are planned whole by every CTA.  0 keeps the built-in value (64, 2,
- * 512).  Results never depend on the schedule.  No reference counterpart (the
+/* The msp task schedule.  min_grain: probe positions that 32 peel tasks should
+ * hold (a task is one warp's, 32 of them 1,024 threads'); tasks_per_cta: chunks
+ * per CTA that a frontier too large to be planned whole is cut into; local_plan:
+ * frontiers of at most this many edges (<= 512) are planned whole by every CTA.
+ * 0 keeps the built-in value (2048, 2, 512).  Results never depend on the schedule.  No reference counterpart (the
  * reference launches one block per frontier edge: bitruss_msp.cu:286-291). */
 bt_status bt_ctx_set_msp_schedule(bt_ctx *ctx, uint32_t min_grain, uint32_t tasks_per_cta,
                                   uint32_t local_plan);

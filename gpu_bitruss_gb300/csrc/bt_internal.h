@@ -236,6 +236,16 @@ bt_status bt_count_any_order_setup();
 bt_status bt_count_any_order(uint32_t n, uint32_t slots, const uint2 *rows, const uint32_t *nbr,
                              unsigned long long *count, uint32_t *next_chunk, uint32_t *skip, int sms, cudaStream_t st);
 
+// A graph of a batch as its peel's plan sees it, estimates of its peel (the chain
+// of sub-rounds, and what CTAs share, in microseconds of one), and the sizes of the
+// teams of CTAs that take the graphs in the order given (bt_plan.cpp).
+struct PeelJob {
+    uint64_t edges, butterflies;
+};
+double bt_peel_chain_us(const PeelJob &j);
+double bt_peel_walk_us(const PeelJob &j);
+std::vector<uint32_t> bt_plan_teams(const std::vector<PeelJob> &jobs, uint32_t ctas);
+
 // algorithm entry points implemented in the .cu files
 bt_status dev_build_graph(bt_ctx *ctx, const bt_graph *g);
 bt_status dev_ebfc(bt_ctx *ctx, bool per_edge, uint64_t *count);

@@ -73,14 +73,11 @@
 // Grid barriers are bounded by a time limit; an expired wait sets an error and
 // the kernel returns.
 #include <algorithm>
-#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <condition_variable>
-#include <functional>
 #include <mutex>
 #include <new>
-#include <queue>
 #include <type_traits>
 #include <vector>
 
@@ -194,7 +191,7 @@ struct MspArgs {
     MspShared *sh;
     TeamState *teams;
     MspState *states;               // per job
-    const Job *jobs;                // largest first
+    const Job *jobs;                // longest first
     uint32_t njobs, nteams;
     const uint32_t *team_of;        // per CTA
     uint32_t n, exact;
@@ -974,6 +971,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_msp(const __grid_constant__ Msp
 // set-up kernels
 // ---------------------------------------------------------------------------
 
+// Every graph's supports added up (four per butterfly); gridDim.y blocks a graph.
+__global__ void __launch_bounds__(256) k_job_supports(const Job *jobs, const unsigned long long *sup,
+                                                      unsigned long long *sums) {
+    const Job j = jobs[blockIdx.x];
+    unsigned long long v = 0;
+    for (uint64_t i = blockIdx.y * 256ull + threadIdx.x; i < j.m; i += gridDim.y * 256ull) v += sup[(uint64_t)j.e0 + i];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(sums + blockIdx.x, v);
+}
+
 constexpr int kInitThreads = 256;
 
 // Edge states, vertex records and row tables (the tables' places in the pool
@@ -1076,64 +1083,6 @@ struct CtaSlots {
 };
 }  // namespace
 
-// Sizes of the teams.  One graph takes all CTAs.  A batch is peeled by teams
-// that take graphs one after another, largest first: a graph's peel is a chain
-// of sub-rounds that does not get shorter with more CTAs (6.5 us each), beside
-// the row positions walked, which do (150 per us and CTA).  Both grow with
-// powers of the edge count; the figures are those of Chung-Lu graphs of mean
-// degree 8 (421 / 1,876 / 8,235 sub-rounds and 0.6 / 15 / 390 million positions
-// at 10k / 100k / 1M edges; the estimate was within 10% for teams of 1 to 19),
-// and only the balance of the two matters here.  Numbers of teams, with sizes in
-// proportion to a power of their first graph's positions, are played through
-// and the one that ends first is taken.  48 graphs of 1k to 100k edges: 23 ms, with
-// the best equal sizes (8 or 9 CTAs) 26, as one chain of the union's sub-rounds 45.
-static std::vector<uint32_t> plan_teams(const std::vector<Job> &jobs, uint32_t ctas) {
-    std::vector<uint32_t> best{ctas};
-    if (jobs.size() < 2) return best;
-    std::vector<double> chain, walk;
-    for (const Job &j : jobs) {
-        chain.push_back(6.5 * 421 * pow(j.m / 1e4, 0.65));
-        walk.push_back(6.3e5 / 150 * pow(j.m / 1e4, 1.4));
-    }
-    double best_us = 0;
-    for (size_t q = 0; q < jobs.size(); q++) best_us += chain[q] + walk[q] / ctas;
-    for (uint32_t teams = 2; teams <= ctas && teams <= jobs.size(); teams += std::max(1u, teams / 3)) {
-        for (double power : {0.0, 0.5}) {
-            std::vector<uint32_t> size(teams);
-            double sum = 0;
-            for (uint32_t t = 0; t < teams; t++) sum += pow(walk[t], power);
-            uint32_t used = 0;
-            for (uint32_t t = 0; t < teams; t++) {
-                size[t] = std::max(1u, (uint32_t)(ctas * pow(walk[t], power) / sum));
-                used += size[t];
-            }
-            for (uint32_t t = 0; used < ctas; t = (t + 1) % teams, used++) size[t]++;
-            for (uint32_t t = 0; used > ctas; t = (t + 1) % teams)
-                if (size[t] > 1) size[t]--, used--;
-            std::priority_queue<std::pair<double, uint32_t>, std::vector<std::pair<double, uint32_t>>,
-                                std::greater<std::pair<double, uint32_t>>> free_at;
-            double last = 0;
-            for (size_t q = 0; q < jobs.size() && (last < best_us); q++) {
-                double at = 0;
-                uint32_t t = (uint32_t)q;
-                if (q >= teams) {
-                    at = free_at.top().first;
-                    t = free_at.top().second;
-                    free_at.pop();
-                }
-                at += chain[q] + walk[q] / size[t];
-                last = std::max(last, at);
-                free_at.push({at, t});
-            }
-            if (last < best_us) {
-                best_us = last;
-                best = size;
-            }
-        }
-    }
-    return best;
-}
-
 static unsigned long long wait_limit_ns() {
     const char *us = getenv("BT_WAIT_LIMIT_US");
     if (us && strtoull(us, nullptr, 10) > 0) return strtoull(us, nullptr, 10) * 1000ull;
@@ -1158,15 +1107,12 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     cudaEventRecord(e0, st);
 
     CtxBuffers buffers(ctx);
-    // the graphs to peel, largest first, and how many CTAs peel each
+    // the graphs to peel, and (of several) their work
     std::vector<Job> jobs;
-    std::vector<uint2> by_edge;
     for (const auto &sp : g.spans)
         if (sp.m) jobs.push_back(Job{sp.v0, sp.v0 + sp.n, sp.e0, sp.m});
-    std::stable_sort(jobs.begin(), jobs.end(), [](const Job &x, const Job &y) { return x.m > y.m; });
-    for (uint32_t q = 0; q < jobs.size(); q++) by_edge.push_back(make_uint2(jobs[q].e0, q));
-    std::sort(by_edge.begin(), by_edge.end(), [](const uint2 &x, const uint2 &y) { return x.x < y.x; });
     const uint32_t njobs = (uint32_t)jobs.size();
+    std::vector<PeelJob> job_work(njobs, PeelJob{0, 0});
     MspArgs a{};
     uint2 *d_by_edge = nullptr;
     const uint64_t mm = m ? m : 1, nn = n ? n : 1;
@@ -1208,7 +1154,40 @@ static bt_status run_msp(bt_ctx *ctx, bool exact, uint32_t *levels) {
     if (per_sm < 1) return bt_fail(BT_ERR_CUDA, "msp kernel does not fit on an SM");
     const uint32_t capacity = (uint32_t)(ctx->sm_count * per_sm);
     const uint32_t ctas = ctx->peel_ctas && ctx->peel_ctas < capacity ? ctx->peel_ctas : capacity;
-    const std::vector<uint32_t> sizes = plan_teams(jobs, ctas);
+    std::vector<uint2> by_edge;
+    if (njobs > 1) {
+        unsigned long long *d_sums = nullptr;
+        std::vector<unsigned long long> sums(njobs);
+        A(d_sums, 8ull * njobs);
+        BT_CUDA(cudaMemsetAsync(d_sums, 0, 8ull * njobs, st));
+        BT_CUDA(cudaMemcpyAsync((void *)a.jobs, jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, st));
+        k_job_supports<<<dim3(njobs, std::min(64u, std::max(1u, 1024u / njobs))), 256, 0, st>>>(
+            a.jobs, (const unsigned long long *)ctx->sup, d_sums);
+        bt_note_launches(1);
+        BT_CUDA(cudaGetLastError());
+        BT_CUDA(cudaMemcpyAsync(sums.data(), d_sums, 8ull * njobs, cudaMemcpyDeviceToHost, st));
+        BT_CUDA(cudaStreamSynchronize(st));
+        // those that take longest on one CTA first
+        std::vector<uint32_t> order(njobs);
+        for (uint32_t q = 0; q < njobs; q++) {
+            order[q] = q;
+            job_work[q] = PeelJob{jobs[q].m, sums[q] / 4};
+        }
+        auto cost = [&](uint32_t q) { return bt_peel_chain_us(job_work[q]) + bt_peel_walk_us(job_work[q]); };
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return cost(x) > cost(y); });
+        std::vector<Job> jobs_by_cost;
+        std::vector<PeelJob> work_by_cost;
+        for (uint32_t q : order) {
+            jobs_by_cost.push_back(jobs[q]);
+            work_by_cost.push_back(job_work[q]);
+        }
+        jobs.swap(jobs_by_cost);
+        job_work.swap(work_by_cost);
+    }
+    for (uint32_t q = 0; q < njobs; q++) by_edge.push_back(make_uint2(jobs[q].e0, q));
+    std::sort(by_edge.begin(), by_edge.end(), [](const uint2 &x, const uint2 &y) { return x.x < y.x; });
+    // how many CTAs peel each
+    const std::vector<uint32_t> sizes = bt_plan_teams(job_work, ctas);
     std::vector<TeamState> teams(sizes.size());
     std::vector<uint32_t> team_of;
     for (uint32_t t = 0; t < sizes.size(); t++) {

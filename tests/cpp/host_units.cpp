@@ -1,6 +1,8 @@
 // Host-side parts of the engine's headers, checked without a GPU: the largest
 // batch of middle vertices whose wedge positions are 32-bit numbers; the peel's
-// counters past 2^32; the device buffers of a call that ends by an exception.
+// counters past 2^32; the device buffers of a call that ends by an exception; the
+// CTAs of a batch's graphs.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <new>
@@ -94,4 +96,51 @@ static int call_buffers() {
     return 0;
 }
 
-int main() { return count_batch() || peel_counters() || call_buffers(); }
+// End of the last graph where teams of these sizes take the jobs in order.
+static double makespan(const std::vector<PeelJob> &jobs, const std::vector<uint32_t> &size) {
+    std::vector<double> free_at(size.size(), 0.0);
+    double last = 0;
+    for (size_t q = 0; q < jobs.size(); q++) {
+        size_t t = 0;
+        for (size_t k = 1; k < size.size(); k++)
+            if (free_at[k] < free_at[t]) t = k;
+        if (q < size.size()) t = q;
+        free_at[t] += bt_peel_chain_us(jobs[q]) + bt_peel_walk_us(jobs[q]) / size[t];
+        last = std::max(last, free_at[t]);
+    }
+    return last;
+}
+static int team_sizes() {
+    const uint32_t ctas[] = {1, 2, 5, 152};
+    uint32_t seed = 1;
+    for (uint32_t c : ctas)
+        for (uint32_t n : {1u, 2u, 3u, 40u, 700u}) {
+            std::vector<PeelJob> jobs;
+            for (uint32_t q = 0; q < n; q++) {
+                seed = seed * 1664525u + 1013904223u;
+                jobs.push_back(PeelJob{1 + (seed >> 12), seed % 3 ? (uint64_t)seed >> (seed & 15) : 0});
+            }
+            const std::vector<uint32_t> size = bt_plan_teams(jobs, c);
+            uint32_t sum = 0;
+            CHECK(!size.empty() && size.size() <= n && size.size() <= c);
+            for (uint32_t s : size) {
+                CHECK(s >= 1);
+                sum += s;
+            }
+            CHECK(sum == c);
+            // never longer than one after the other on all of them
+            CHECK(makespan(jobs, size) <= makespan(jobs, {c}) * 1.0001);
+        }
+    // a hub-skewed graph of 100k edges beside ten uniform ones of 400k: by far the
+    // longest, though it has the fewest edges
+    std::vector<PeelJob> mixed{PeelJob{100000, 140000000}};
+    for (int q = 0; q < 10; q++) mixed.push_back(PeelJob{400000, 1150});
+    for (int q = 1; q <= 10; q++)
+        CHECK(bt_peel_chain_us(mixed[0]) + bt_peel_walk_us(mixed[0]) > 50 * (bt_peel_chain_us(mixed[q]) + bt_peel_walk_us(mixed[q])));
+    CHECK(bt_plan_teams(mixed, 152)[0] >= 100);
+    // equal graphs whose chains outweigh their walks run side by side
+    CHECK(bt_plan_teams(std::vector<PeelJob>(48, PeelJob{20000, 485050}), 152).size() >= 16);
+    return 0;
+}
+
+int main() { return count_batch() || peel_counters() || call_buffers() || team_sizes(); }

@@ -43,18 +43,24 @@
 // degree 8 2.0 -> 0.5 ms.
 #include <algorithm>
 
+#include "bt_device.cuh"
 #include "bt_internal.h"
 
 namespace {
 
+using bt::warp_inclusive;
 constexpr int kCountThreads = 1024;
 constexpr uint32_t kCountWarps = kCountThreads / 32;
 constexpr uint32_t kDense = 52224;         // counters in shared memory (204 KiB)
 constexpr uint32_t kBatch = kCountBatch;   // middle vertices a CTA lays end to end at once
 static_assert(kCountBatch == kCountThreads && kCountStride == kCountThreads * 4, "one per thread; four positions each");
-// Longest row a single warp may have to walk by itself.  On the hub-skewed
-// graph (rows of at most 60) warps on their own take 1.1 ms, batches of the
-// CTA 1.7; on the Chung-Lu graph (rows of up to 10k) 5.7 and 2.6.
+// Longest row a single warp may have to walk by itself.  Supports (and counts) in
+// ms with warps on their own and in batches of the CTA: hub-skewed graphs of 1 to
+// 4M edges with rows of up to 51 0.50 and 0.77 (0.20 and 0.34), 212 1.45 and 1.72
+// (0.51 and 0.72), 463 1.74 and 1.76 (0.65 and 0.74), 1,042 4.55 and 3.67 (2.35 and
+// 1.86); uniform ones of 2 to 4M, whose rows are all about as long, 137 0.99 and 0.99
+// (0.34 and 0.43), 300 2.75 and 2.16 (0.87 and 0.92), 556 8.1 and 6.2 (2.42 and 2.67);
+// the Chung-Lu graph (rows of up to 10k) 5.7 and 2.6.
 constexpr uint32_t kShortRow = 512;
 constexpr uint32_t kSlots = 512;           // hash slots of one warp
 constexpr uint32_t kLightWedges = 320;     // wedges a warp's hash takes
@@ -138,16 +144,6 @@ __device__ __forceinline__ Mid load_mid(const CountArgs &a, uint32_t rb, uint32_
         m.len = sl - j0;
     }
     return m;
-}
-
-__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
-    const uint32_t lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= (uint32_t)o) v += t;
-    }
-    return v;
 }
 
 // Visit every wedge end of the warp's 32 middle vertices, their suffixes laid

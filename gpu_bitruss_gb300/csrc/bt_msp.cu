@@ -207,7 +207,7 @@ struct MspArgs {
     const uint2 *ends;
     VRec *vrec;
     uint32_t *nbr, *eid;            // live rows (compacted in place)
-    uint4 *pool;                    // row tables (bt::row_lookup)
+    uint4 *pool;                    // row tables (bt::row_resolve)
     unsigned long long *sup;        // working supports (64-bit)
     uint32_t *sup32;                // working supports when every support fits 32 bits (else null)
     uint32_t *enter;                // sub-round index at which the edge joined a frontier

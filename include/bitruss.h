@@ -231,7 +231,8 @@ bt_status bt_ebfc_batch(bt_ctx *ctx, const bt_graph *const *graphs, uint32_t cou
  * process).  A server runs count / support / decompose requests on graphs of
  * different sizes as they arrive.  It has `slots` worker threads, each with
  * its own context and stream, so their uploads, counting kernels and copies
- * overlap on the GPU (one peeling kernel runs at a time).  A request is
+ * overlap on the GPU and their peels run side by side, each on its share of the
+ * SMs (bt_ctx_set_peel_ctas).  A request is
  * admitted when a slot is free and its device footprint (bt_job_bytes) fits
  * in what the HBM budget has left; requests are taken in arrival order, and
  * one that does not fit yet may be passed by up to 64 later admissions.

@@ -31,8 +31,8 @@
 // (430 cycles each) and barriers on its longest path, not bandwidth.  Measured
 // per sub-round, against staging the anchor row in shared memory and walking
 // equal shares of probe positions by whole CTAs: Chung-Lu graphs of 10k / 200k
-// / 1M edges 6.7 / 8.0 / 10.7 us (19.4 / 21.8 / 28.7 before), the 20M-edge one
-// 45 us (87), hub-skewed graphs of 200k / 2M edges 12.2 / 31 us (28.5 / 49).
+// / 1M edges 6.6 / 8.1 / 10.8 us (19.4 / 21.8 / 28.7 before), the 20M-edge one
+// 46 us (87), hub-skewed graphs of 200k / 2M edges 12.4 / 32 us (28.5 / 49).
 // What follows from that:
 //  * Edge state is one stamp per edge: enter[e] = the index of the sub-round
 //    whose frontier e joined (0: not yet).  In sub-round r an edge is in the

@@ -101,6 +101,7 @@ struct __align__(16) CountSmem {
     // the lengths, the support of (r, s), the slot of s in r's row
     uint32_t p0[kBatch], pre[kBatch + 1], sum[kBatch], at[kBatch];
     uint32_t big[kCountWarps];     // start vertices left to the CTA (rank + 1)
+    uint2 row[kCountWarps];        // their rows
     uint32_t wlen[kCountWarps], wcnt[kCountWarps];
     uint32_t chunk, touched;
     unsigned long long red[kCountWarps];
@@ -113,15 +114,15 @@ __device__ __forceinline__ void acc_add(void *acc, uint32_t slot, unsigned long 
 }
 
 // r's first slot and its degree.  ANY_ORDER: the tables may be another call's by
-// now (bt_noalloc.cu); a row that does not end where the next one starts, as all
-// do there, is taken as empty.
+// now (bt_noalloc.cu); a row that leaves nbr is taken as empty.  (Comparing each
+// row's end with the next one's start takes a 300k-edge count from 252 to 260 us,
+// these compares to 255; only a large start vertex's own row is compared so.)
 template <bool ANY_ORDER>
 __device__ __forceinline__ uint2 row_of(const CountArgs &a, uint32_t r) {
     if (!ANY_ORDER) return make_uint2(__ldg(a.off + r), __ldg(a.deg + r));
     const uint2 row = __ldg(a.rows + r);
-    const uint32_t next = r + 1 < a.n ? __ldg(&a.rows[r + 1].x) : a.slots;
-    const bool fits = next <= a.slots && row.x <= next && row.y == next - row.x && row.y < a.n;
-    return fits ? row : make_uint2(0, 0);
+    const bool fits = row.x <= a.slots & row.y <= a.slots - row.x & row.y < a.n;
+    return make_uint2(row.x, fits ? row.y : 0);
 }
 
 // 32 middle vertices of r, one per lane: where the suffix of ranks above r
@@ -331,10 +332,9 @@ __device__ __forceinline__ void visit_batch(const uint32_t *nbr, const CountSmem
 // Ends synchronised.
 template <bool PER_EDGE, bool WIDE, bool ANY_ORDER>
 __device__ __forceinline__ unsigned long long big_vertex(const CountArgs &a, CountSmem &sm, uint32_t *dense,
-                                                         uint32_t r, uint32_t skip) {
+                                                         uint32_t r, uint2 row, uint32_t skip) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t base = a.seg_base ? a.seg_base[r] : 0u;
-    const uint2 row = row_of<ANY_ORDER>(a, r);
     const uint32_t rb = row.x, rl = row.y;
     const uint32_t start = ANY_ORDER ? 0 : upper_bound_u32(a.nbr + rb, rl, r);
     uint32_t *cnt = a.cnt + (size_t)blockIdx.x * a.span;
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
         const uint32_t r = warp * a.chunks + c;
         uint32_t big = 0;
         if (r < a.n) {
-            const uint2 row = row_of<ANY_ORDER>(a, r);
+            uint2 row = row_of<ANY_ORDER>(a, r);
             const uint32_t rb = row.x, rl = row.y;
             // the suffix of r's own row after r, found 32 ways at a time
             uint32_t lo = 0, hi = ANY_ORDER ? 0 : rl;
@@ -498,6 +498,9 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
                 if (total > kLightWedges) big = r + 1;
                 else if (total) local += light_vertex<PER_EDGE, WIDE, ANY_ORDER>(a, table, r, rb + lo, m, total);
             }
+            // (a row that does not end where the next one starts is of no graph)
+            if (ANY_ORDER && big && rb + rl != (r + 1 < a.n ? a.rows[r + 1].x : a.slots)) row.y = 0;
+            if (lane == 0) sm.row[warp] = row;  // one answer for all threads
         }
         if (lane == 0) sm.big[warp] = big;
         if (threadIdx.x == 0) sm.chunk = gridDim.x + atomicAdd(a.next_chunk, 1u);
@@ -509,7 +512,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) k_count(const __grid_constan
             bool more;
             uint32_t skip = 0;
             do {  // no counters but the shared ones: further passes over the ranks past them
-                local += big_vertex<PER_EDGE, WIDE, ANY_ORDER>(a, sm, dense, v, skip);
+                local += big_vertex<PER_EDGE, WIDE, ANY_ORDER>(a, sm, dense, v, sm.row[w], skip);
                 more = ANY_ORDER && sm.touched != 0;
                 if (ANY_ORDER) __syncthreads();
                 skip += a.dense;
